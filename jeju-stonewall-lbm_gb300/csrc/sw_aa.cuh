@@ -67,7 +67,15 @@ __device__ __forceinline__ typename Store<DT>::R aa_ld(const typename Store<DT>:
   else return *q;                                           // coherent loads: the lattice is written in place
 }
 
+// A float64 cell stepped in place with the collision in double, without its wall
+// force (see step_cell_double): nothing of the cell is written yet, and what it
+// pulls is written by no other cell.
 template <int DT, bool CHECK, bool ACC>
+__device__ __noinline__ void aa_odd_cell_double(const StepParams &p, const AAParams &a, int x, int y, int z);
+template <int DT, bool CHECK, bool ACC>
+__device__ __noinline__ void aa_even_cell_double(const StepParams &p, int x, int y, int z);
+
+template <int DT, bool CHECK, bool ACC, bool FIXED = DT == SW_F64>
 __device__ __forceinline__ void aa_odd_cell(const StepParams &p, const AAParams &a, int x, int y, int z,
                                             typename Store<DT>::R &fxw, typename Store<DT>::R &fzw, int &hit) {
   using S = Store<DT>;
@@ -184,9 +192,13 @@ __device__ __forceinline__ void aa_odd_cell(const StepParams &p, const AAParams 
     });
     rho = R(1.0); ux = u0; uy = R(0.0); uz = R(0.0);
   } else {
-    const Phys<R> ph = phys<R>(p);
-    collide<R, S::kShift>(fl, x, ph.nu0, ph.c18, p.x_sponge, ph.sponge_scale, ph.nu_sponge, rho, ux, uy, uz,
-                          p.status, scatter);
+    const bool done = collide_cell<R, S::kShift, ACC, FIXED>(p, fl, x, rho, ux, uy, uz, scatter);
+    if constexpr (FIXED) {
+      if (!done) {
+        aa_odd_cell_double<DT, CHECK, ACC>(p, a, x, y, z);
+        return;
+      }
+    }
   }
   if (ACC) {
     atomicAdd(p.accp(0) + c, (double)rho);
@@ -196,7 +208,7 @@ __device__ __forceinline__ void aa_odd_cell(const StepParams &p, const AAParams 
   }
 }
 
-template <int DT, bool CHECK, bool ACC>
+template <int DT, bool CHECK, bool ACC, bool FIXED = DT == SW_F64>
 __device__ __forceinline__ void aa_even_cell(const StepParams &p, int x, int y, int z, typename Store<DT>::R &fxw,
                                              typename Store<DT>::R &fzw, int &hit) {
   using S = Store<DT>;
@@ -252,9 +264,13 @@ __device__ __forceinline__ void aa_even_cell(const StepParams &p, int x, int y, 
         }
       });
     }
-    const Phys<R> ph = phys<R>(p);
-    collide<R, S::kShift>(fl, x, ph.nu0, ph.c18, p.x_sponge, ph.sponge_scale, ph.nu_sponge, rho, ux, uy, uz,
-                          p.status, put);
+    const bool done = collide_cell<R, S::kShift, ACC, FIXED>(p, fl, x, rho, ux, uy, uz, put);
+    if constexpr (FIXED) {
+      if (!done) {
+        aa_even_cell_double<DT, CHECK, ACC>(p, x, y, z);
+        return;
+      }
+    }
   }
   if (ACC) {
     atomicAdd(p.accp(0) + c, (double)rho);
@@ -262,6 +278,19 @@ __device__ __forceinline__ void aa_even_cell(const StepParams &p, int x, int y, 
     atomicAdd(p.accp(2) + c, (double)uy);
     atomicAdd(p.accp(3) + c, (double)uz);
   }
+}
+
+template <int DT, bool CHECK, bool ACC>
+__device__ __noinline__ void aa_odd_cell_double(const StepParams &p, const AAParams &a, int x, int y, int z) {
+  typename Store<DT>::R fxw(0), fzw(0);
+  int hit = 0;
+  aa_odd_cell<DT, CHECK, ACC, false>(p, a, x, y, z, fxw, fzw, hit);
+}
+template <int DT, bool CHECK, bool ACC>
+__device__ __noinline__ void aa_even_cell_double(const StepParams &p, int x, int y, int z) {
+  typename Store<DT>::R fxw(0), fzw(0);
+  int hit = 0;
+  aa_even_cell<DT, CHECK, ACC, false>(p, x, y, z, fxw, fzw, hit);
 }
 
 template <int DT, bool ODD, bool ACC, typename Cfg>
@@ -672,13 +701,14 @@ cudaError_t launch_aa(const StepParams &p_in, const AAParams &a, bool odd, cudaS
   StepParams p = p_in;
   set_plane_bases(p, sizeof(T));                    // fin == fout == the lattice: natural plane bases
   set_float_params(p);
+  set_double_params(p);
   const size_t pb = (size_t)p.g.plane * sizeof(T);
   for (int i = 0; i < Q; ++i) {
     if (odd) p.fout_pop[i] = static_cast<char *>(p.fout) + (size_t)OPP(i) * pb;
     else p.fin_pop[i] = static_cast<const char *>(p.fin) + (size_t)OPP(i) * pb;
   }
   using C3 = StepCfg<4, 12>;
-  using C0 = StepCfg<8, 4>;
+  using C0 = StepCfgOf<SW_F64, 4, 8>;
   if (odd) {
     const dim3 gg((unsigned)((p.g.ny + 127) / 128), (unsigned)p.g.nz);
     k_aa_ghost<DT><<<gg, 128, 0, s>>>(p, a);
@@ -718,7 +748,7 @@ cudaError_t launch_aa(const StepParams &p_in, const AAParams &a, bool odd, cudaS
     }
     return cudaGetLastError();
   };
-  if constexpr (DT == SW_F64) return go(C0{});      // float64 registers: the wide, low-occupancy shape
+  if constexpr (DT == SW_F64) return go(C0{});      // the registers of the float64 populations
   else return go(C3{});
 }
 

@@ -27,6 +27,7 @@ struct BatchCtx {
   const float *uin;
   double nu0, cs, nu_sponge, sponge_scale;
   float nu0f, c18f, sponge_scalef, nu_spongef;   // as StepParams (set_float_params)
+  double c18, tau0, tau0sq;                      // as StepParams (set_double_params)
   int x_sponge;
   long long *force;
   unsigned int *status;     // the lattice's status word, or nullptr
@@ -126,6 +127,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
           sc.c18f = smag_c18f((float)e.cs);
           sc.sponge_scalef = (float)sc.sponge_scale;
           sc.nu_spongef = (float)e.nu_sponge;
+          if constexpr (DT == SW_F64) set_double_params(sc);
           sc.status = e.status;
           const long long t = e.t0 + k;
           sc.force = e.force ? reinterpret_cast<long long *>(e.force) + t * 2 * e.geom.nz : nullptr;
@@ -193,7 +195,7 @@ template <int DT>
 cudaError_t launch_batch(const sw_batch_header *hdr, const sw_batch_entry *tab, int cfg, int k, cudaStream_t s) {
   switch (cfg) {
 #define SW_CASE(ID, WY, MINB) \
-  case ID: return launch_batch_cfg<DT, false, StepCfg<WY, MINB>>(hdr, tab, k, s);
+  case ID: return launch_batch_cfg<DT, false, StepCfgOf<DT, WY, MINB>>(hdr, tab, k, s);
     SW_STEP_CONFIGS(SW_CASE)
 #undef SW_CASE
 #define SW_CASE(ID, WY, MINB)                                                     \

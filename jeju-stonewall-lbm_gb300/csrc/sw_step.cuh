@@ -28,6 +28,7 @@
 //    n_acc * (1, 0, 0, 0) by definition and are filled in on download.
 #pragma once
 #include "sw_common.cuh"
+#include "sw_f64.cuh"
 
 namespace sw {
 
@@ -43,6 +44,8 @@ struct StepParams {
   // float copies for the float collision (set_float_params): rounded once on
   // the host instead of converted from double in every thread
   float nu0f, c18f, sponge_scalef, nu_spongef;
+  // the same for the float64 collision: 18 sqrt(2) Cs^2, 3 nu0 + 1/2 and its square (set_double_params)
+  double c18, tau0, tau0sq;
   int x_sponge;
   long long *force;  // force row of this step: [nz][2], or nullptr
   double *acc;       // float64 running sums [4][plane] (accumulation steps only)
@@ -90,17 +93,20 @@ inline void set_float_params(StepParams &p) {
   p.nu_spongef = (float)p.nu_sponge;
 }
 
+// The float64 collision's parameters (StepParams on the host, the batched kernel's context on the device).
+template <typename P> __host__ __device__ inline void set_double_params(P &p) {
+  p.c18 = 18.0 * sqrt(2.0) * p.cs * p.cs;
+  p.tau0 = fma(3.0, p.nu0, 0.5);
+  p.tau0sq = p.tau0 * p.tau0;
+}
+
 // Physics parameters in the collision's arithmetic type R.
 template <typename R> struct Phys {
   R nu0, c18, sponge_scale, nu_sponge;
 };
 template <typename R, typename Ctx> __device__ __forceinline__ Phys<R> phys(const Ctx &p) {
-  if constexpr (sizeof(R) == 4) {
-    return {p.nu0f, p.c18f, p.sponge_scalef, p.nu_spongef};
-  } else {
-    const R cs = p.cs;
-    return {p.nu0, R(18.0) * sqrt(R(2.0)) * cs * cs, p.sponge_scale, p.nu_sponge};
-  }
+  if constexpr (sizeof(R) == 4) return {p.nu0f, p.c18f, p.sponge_scalef, p.nu_spongef};
+  else return {p.nu0, p.c18, p.sponge_scale, p.nu_sponge};
 }
 
 // ORs status bits into the lattice's status word (a rare branch: divergence or a time-out).
@@ -225,6 +231,38 @@ __device__ __forceinline__ void collide(const R (&f)[Q], int x, R nu0, R cs2_18r
   uz_out = uz;
 }
 
+// The collision of a cell of a step kernel: as collide, with the parameters of
+// the kernel's context.  FIXED (float64 storage): in fixed point (sw_f64.cuh);
+// false when the cell is out of its range, before anything is put, and the
+// caller steps the cell again without FIXED.  WANT: rho and u are used.
+template <typename R, bool SHIFT, bool WANT, bool FIXED, typename Ctx, typename Put>
+__device__ __forceinline__ bool collide_cell(const Ctx &p, const R (&f)[Q], int x, R &rho, R &ux, R &uy, R &uz,
+                                             Put &&put) {
+  const Phys<R> ph = phys<R>(p);
+  if constexpr (!FIXED) {
+    collide<R, SHIFT>(f, x, ph.nu0, ph.c18, p.x_sponge, ph.sponge_scale, ph.nu_sponge, rho, ux, uy, uz, p.status, put);
+  } else {
+    static_assert(!SHIFT && sizeof(R) == 8, "fixed point takes float64 storage, which holds f itself");
+    double tau0 = p.tau0, tau0sq = p.tau0sq;
+    if (x > p.x_sponge) {
+      const double sp = (double)(x - p.x_sponge) * ph.sponge_scale;
+      tau0 = fma(3.0, fma(ph.nu_sponge * sp, sp, ph.nu0), 0.5);
+      tau0sq = tau0 * tau0;
+    }
+    double out[Q];
+    fx::Moments m;
+    if (!fx::collide(f, tau0, tau0sq, ph.c18, out, m)) return false;
+    static_for<0, Q>([&](auto I) { put(I, out[decltype(I)::value]); });
+    if constexpr (WANT) {
+      rho = m.rho();
+      ux = m.vel(0);
+      uy = m.vel(1);
+      uz = m.vel(2);
+    }
+  }
+  return true;
+}
+
 // Launch configurations compiled in; the autotuner (stonewall/autotune.py)
 // times them per storage type and grid and keeps the fastest.
 //   WY   rows of a block (one 32-cell segment per warp): block = 32 x WY threads
@@ -235,6 +273,10 @@ template <int WY_, int MINB_> struct StepCfg {
   static constexpr int THREADS = 32 * WY_;
 };
 #define SW_STEP_CONFIGS(X) X(0, 8, 4) X(1, 8, 5) X(2, 4, 8) X(3, 4, 12)
+// The float64 step holds its 19 populations in register pairs: the same block
+// shapes with the registers that takes (128, 80, 96 and 80 per thread).
+template <int DT, int WY, int MINB>
+using StepCfgOf = StepCfg<WY, DT != SW_F64 ? MINB : WY == 8 ? (MINB == 4 ? 2 : 3) : (MINB == 8 ? 5 : 6)>;
 // two cells per thread (16-bit storage only), see k_step_pair
 #define SW_PAIR_CONFIGS(X) X(4, 4, 8) X(5, 4, 10) X(6, 8, 4) X(7, 8, 5)
 // two cells per thread with TMA-staged sources (16-bit storage only), see sw_tma.cuh:
@@ -276,6 +318,12 @@ template <int DT> struct GlobalPull {
   }
 };
 
+// A float64 cell stepped with the collision in double, without its wall force (a
+// separate function: such cells are rare, and inlined it would keep the pulled
+// values of every cell live to the end).
+template <int DT, bool CHECK, bool ACC, typename Ctx>
+__device__ __noinline__ void step_cell_double(const Ctx &p, int x, int y, int z);
+
 // One cell of the pull-scheme step.  CHECK selects the path with neighbour flag
 // tests (segments next to stones, the ground or a fluid cell at z = 0).
 // Offsets within a population plane are 32-bit (grids below 2^31 cells).
@@ -287,7 +335,9 @@ __device__ __forceinline__ void step_cell(const Ctx &p, int x, int y, int z, typ
 
 // The same with the checked path's inputs from `pull_val` (GlobalPull: the
 // lattice and the flags).
-template <int DT, bool CHECK, bool ACC, typename Ctx, typename Pull>
+// FIXED: float64 storage collides in fixed point and hands the few cells out of
+// its range to step_cell_double.
+template <int DT, bool CHECK, bool ACC, bool FIXED = DT == SW_F64, typename Ctx, typename Pull>
 __device__ __forceinline__ void step_cell(const Ctx &p, int x, int y, int z, typename Store<DT>::R &fxw,
                                           typename Store<DT>::R &fzw, int &hit, const Pull &pull_val) {
   using S = Store<DT>;
@@ -363,18 +413,29 @@ __device__ __forceinline__ void step_cell(const Ctx &p, int x, int y, int z, typ
     }
   });
   R rho, ux, uy, uz;
-  const Phys<R> ph = phys<R>(p);
-  collide<R, S::kShift>(fl, x, ph.nu0, ph.c18, p.x_sponge, ph.sponge_scale, ph.nu_sponge, rho, ux, uy, uz, p.status,
-                        [&](auto I, R v) {
-                          constexpr int i = decltype(I)::value;
-                          S::template st<i>(out(i) + c, v);
-                        });
+  const bool done = collide_cell<R, S::kShift, ACC, FIXED>(p, fl, x, rho, ux, uy, uz, [&](auto I, R v) {
+    constexpr int i = decltype(I)::value;
+    S::template st<i>(out(i) + c, v);
+  });
+  if constexpr (FIXED) {
+    if (!done) {                                                // nothing written yet; the force is summed already
+      step_cell_double<DT, CHECK, ACC>(p, x, y, z);
+      return;
+    }
+  }
   if (ACC) {
     __stcs(p.accp(0) + c, acc_old[0] + (double)rho);
     __stcs(p.accp(1) + c, acc_old[1] + (double)ux);
     __stcs(p.accp(2) + c, acc_old[2] + (double)uy);
     __stcs(p.accp(3) + c, acc_old[3] + (double)uz);
   }
+}
+
+template <int DT, bool CHECK, bool ACC, typename Ctx>
+__device__ __noinline__ void step_cell_double(const Ctx &p, int x, int y, int z) {
+  typename Store<DT>::R fxw(0), fzw(0);
+  int hit = 0;
+  step_cell<DT, CHECK, ACC, false>(p, x, y, z, fxw, fzw, hit, GlobalPull<DT>{});
 }
 
 // Adds the warp's wall force (lbm3d.py:99-101): float64 xor-butterfly sum, then
@@ -946,10 +1007,12 @@ cudaError_t launch_step(const StepParams &p_in, cudaStream_t s) {
   StepParams p = p_in;
   set_plane_bases(p, sizeof(typename Store<DT>::T));
   set_float_params(p);
+  set_double_params(p);
   switch (p.cfg) {
 #define SW_CASE(ID, WY, MINB)                                                                      \
   case ID:                                                                                         \
-    return p.acc ? launch_cfg<DT, true, StepCfg<WY, MINB>>(p, s) : launch_cfg<DT, false, StepCfg<WY, MINB>>(p, s);
+    return p.acc ? launch_cfg<DT, true, StepCfgOf<DT, WY, MINB>>(p, s)                                     \
+                 : launch_cfg<DT, false, StepCfgOf<DT, WY, MINB>>(p, s);
     SW_STEP_CONFIGS(SW_CASE)
 #undef SW_CASE
 #define SW_CASE(ID, WY, MINB)                                                                      \
