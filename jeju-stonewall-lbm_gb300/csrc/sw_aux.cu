@@ -33,42 +33,93 @@ __device__ __forceinline__ float gauss_pair(uint32_t &st, float *second) {
   return r * cs;
 }
 
-// k_init, lbm3d.py:39-54.  One thread per cell of the padded grid.
-template <int DT>
-__global__ void k_init(Geom g, typename Store<DT>::T *f, const uint8_t *flag, const float *uin, float noise,
-                       int seed, int noise_kind) {
-  using S = Store<DT>;
-  using R = typename S::R;
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= g.plane) return;
-  const int x = (int)(c % g.pitch);
-  const long long row = c / g.pitch;
-  const int y = (int)(row % g.ny), z = (int)(row / g.ny);
-  if (x >= g.nx) return;
-  R ux = R(0.0), uy = R(0.0), uz = R(0.0);
-  if (flag[c] == 0) {
-    const uint32_t off = ((uint32_t)x * 7919u + (uint32_t)y) * 7907u + (uint32_t)z;
-    uint32_t st = pcg_hash((uint32_t)seed + pcg_hash(off));
-    const R u0 = (R)uin[z];
-    const R nz_ = (R)noise;
-    if (noise_kind == SW_NOISE_UNIFORM) {
-      ux = u0 * (R(1.0) + nz_ * (R(2.0) * (R)randf(st) - R(1.0)));
-      uy = u0 * nz_ * (R(2.0) * (R)randf(st) - R(1.0));
-      uz = u0 * nz_ * (R(2.0) * (R)randf(st) - R(1.0));
-    } else {
-      float g2 = 0.0f;
-      const float g1 = gauss_pair(st, &g2);
-      const float g3 = gauss_pair(st, nullptr);
-      ux = u0 * (R(1.0) + nz_ * (R)g1);
-      uy = u0 * nz_ * (R)g2;
-      uz = u0 * nz_ * (R)g3;
-    }
+// Velocity of k_init at a cell (lbm3d.py:45-52): the perturbed inlet speed, rest at solids.
+template <typename R>
+__device__ __forceinline__ void init_velocity(bool fluid, int x, int y, int z, const float *uin, float noise, int seed,
+                                              int noise_kind, R &ux, R &uy, R &uz) {
+  ux = uy = uz = R(0.0);
+  if (!fluid) return;
+  const uint32_t off = ((uint32_t)x * 7919u + (uint32_t)y) * 7907u + (uint32_t)z;
+  uint32_t st = pcg_hash((uint32_t)seed + pcg_hash(off));
+  const R u0 = (R)uin[z];
+  const R nz_ = (R)noise;
+  if (noise_kind == SW_NOISE_UNIFORM) {
+    ux = u0 * (R(1.0) + nz_ * (R(2.0) * (R)randf(st) - R(1.0)));
+    uy = u0 * nz_ * (R(2.0) * (R)randf(st) - R(1.0));
+    uz = u0 * nz_ * (R(2.0) * (R)randf(st) - R(1.0));
+  } else {
+    float g2 = 0.0f;
+    const float g1 = gauss_pair(st, &g2);
+    const float g3 = gauss_pair(st, nullptr);
+    ux = u0 * (R(1.0) + nz_ * (R)g1);
+    uy = u0 * nz_ * (R)g2;
+    uz = u0 * nz_ * (R)g3;
   }
+}
+
+// feq_i (lbm3d.py:33-36) at rho = 1 for all populations, in feq_i's order for
+// each: put(Int<i>, value).  The terms of c_a = 0 are left out (they add a zero)
+// and the members of a pair share (c.u)^2.
+template <typename R, typename Put>
+__device__ __forceinline__ void init_populations(R ux, R uy, R uz, Put &&put) {
+  const R k = R(1.5) * (ux * ux + uy * uy + uz * uz);
+  put(Int<0>{}, W<R>(0) * ((R(1.0) + R(0.0)) - k));
+  static_for<0, 9>([&](auto P) {
+    constexpr int i = 2 * decltype(P)::value + 1;
+    constexpr int cx = CX(i), cy = CY(i), cz = CZ(i);
+    R cu;
+    if constexpr (cx != 0 && cy != 0) cu = (cx > 0 ? ux : -ux) + (cy > 0 ? uy : -uy);
+    else if constexpr (cx != 0 && cz != 0) cu = (cx > 0 ? ux : -ux) + (cz > 0 ? uz : -uz);
+    else if constexpr (cy != 0 && cz != 0) cu = (cy > 0 ? uy : -uy) + (cz > 0 ? uz : -uz);
+    else if constexpr (cx != 0) cu = cx > 0 ? ux : -ux;
+    else if constexpr (cy != 0) cu = cy > 0 ? uy : -uy;
+    else cu = cz > 0 ? uz : -uz;
+    cu = R(3.0) * cu;
+    const R h = R(0.5) * cu * cu;
+    put(Int<i>{}, W<R>(i) * (R(1.0) + cu + h - k));
+    put(Int<i + 1>{}, W<R>(i) * (R(1.0) - cu + h - k));
+  });
+}
+
+// k_init, lbm3d.py:39-54.  CPT cells per thread along x: two in the 16-bit types,
+// stored as one 32-bit word a population.  Bound by the stores and, with
+// Gaussian noise, as much by its logarithms and sines; 32-bit index arithmetic
+// (a plane has fewer than 2^31 cells) and the shared pair terms took a
+// 640x128x128 fp16 lattice from 173 to 137 us.
+template <int DT, int CPT>
+__global__ void __launch_bounds__(256) k_init(Geom g, typename Store<DT>::T *f, const uint8_t *flag, const float *uin,
+                                              float noise, int seed, int noise_kind) {
+  using S = Store<DT>;
+  using T = typename S::T;
+  using R = typename S::R;
+  const uint32_t c = (blockIdx.x * 256u + threadIdx.x) * CPT;
+  if (c >= (uint32_t)g.plane) return;
+  const uint32_t row = c / (uint32_t)g.pitch;
+  const int x = (int)(c - row * (uint32_t)g.pitch);
+  const int z = (int)(row / (uint32_t)g.ny), y = (int)(row - (uint32_t)z * (uint32_t)g.ny);
+  if (x >= g.nx) return;
   const size_t plane = (size_t)g.plane;
+  T v[CPT][Q];
+#pragma unroll
+  for (int j = 0; j < CPT; ++j) {
+    R ux, uy, uz;
+    init_velocity<R>(x + j < g.nx && flag[c + j] == 0, x + j, y, z, uin, noise, seed, noise_kind, ux, uy, uz);
+    init_populations<R>(ux, uy, uz, [&](auto I, R w) {
+      constexpr int i = decltype(I)::value;
+      v[j][i] = S::template enc<i>(w);
+    });
+  }
   static_for<0, Q>([&](auto I) {
     constexpr int i = decltype(I)::value;
-    const R v = feq_i<R>(W<R>(i), R(CX(i)), R(CY(i)), R(CZ(i)), R(1.0), ux, uy, uz);
-    f[(size_t)i * plane + c] = S::template enc<i>(v);
+    T *o = f + (size_t)i * plane + c;
+    if constexpr (CPT == 2) {
+      if (x + 1 < g.nx) {
+        struct alignas(2 * sizeof(T)) Pair { T a, b; };
+        *reinterpret_cast<Pair *>(o) = Pair{v[0][i], v[1][i]};
+        return;
+      }
+    }
+    *o = v[0][i];
   });
 }
 
@@ -110,43 +161,84 @@ __global__ void k_accum(Geom g, const float *u, double *acc) {
   acc[c] += (double)u[c];
 }
 
+// The 32 flags of a row segment as bit masks: not fluid, and stone.
+struct SegMask {
+  uint32_t solid, wall;
+};
+// bit k of the result: byte k of w is not zero
+__device__ __forceinline__ uint32_t nonzero_bytes(uint32_t w) {
+  const uint32_t t = ((((w & 0x7f7f7f7fu) + 0x7f7f7f7fu) | w) >> 7) & 0x01010101u;
+  return (t * 0x10204080u) >> 28;
+}
+template <bool ALIGNED> __device__ __forceinline__ SegMask seg_mask(const uint8_t *seg) {
+  uint32_t w[8];
+  if constexpr (ALIGNED) {
+    const uint4 a = __ldg(reinterpret_cast<const uint4 *>(seg)), b = __ldg(reinterpret_cast<const uint4 *>(seg) + 1);
+    w[0] = a.x, w[1] = a.y, w[2] = a.z, w[3] = a.w, w[4] = b.x, w[5] = b.y, w[6] = b.z, w[7] = b.w;
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      w[k] = seg[4 * k] | (uint32_t)seg[4 * k + 1] << 8 | (uint32_t)seg[4 * k + 2] << 16 | (uint32_t)seg[4 * k + 3] << 24;
+  }
+  SegMask m{0u, 0u};
+  if (((w[0] | w[1]) | (w[2] | w[3])) | ((w[4] | w[5]) | (w[6] | w[7]))) {   // (most segments are all fluid)
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      m.solid |= nonzero_bytes(w[k]) << (4 * k);
+      m.wall |= (nonzero_bytes(w[k] ^ 0x01010101u) ^ 15u) << (4 * k);
+    }
+  }
+  return m;
+}
+
 // Segment classification for the step kernel (see TILE_* in sw_common.cuh).
-// Mirrors the pull-source mapping of the step (lbm3d.py:77-88).
-__global__ void k_build_tiles(Geom g, const uint8_t *flag, uint8_t *tiles) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long nseg = (long long)g.nseg_x * g.ny * g.nz;
-  const long long seg = c >> 5;
-  if (seg >= nseg) return;  // whole warps only (plane is a multiple of 32)
-  const int lane = threadIdx.x & 31;
-  const int x = (int)(c % g.pitch);
-  const long long row = c / g.pitch;
-  const int y = (int)(row % g.ny), z = (int)(row / g.ny);
-  const bool live = x < g.nx;
-  bool fluid = false, nonfluid_src = false, wall_src = false;
-  if (live) {
-    fluid = flag[c] == 0;
-    if (fluid && x > 0) {  // inlet cells do not pull
-      const int ym = (y == 0) ? g.ny - 1 : y - 1, yp = (y == g.ny - 1) ? 0 : y + 1;
-      const int zp = (z == g.nz - 1) ? z : z + 1;
-      const int xp = (x + 1 >= g.nx) ? x : x + 1;
-      for (int i = 1; i < Q; ++i) {
-        const int ex = CX(i), ey = CY(i), ez = CZ(i);
-        if (ez == 1 && z == 0) { nonfluid_src = true; continue; }
-        const int xs = ex == 1 ? x - 1 : (ex == -1 ? xp : x);
-        const int ys = ey == 1 ? ym : (ey == -1 ? yp : y);
-        const int zs = ez == 1 ? z - 1 : (ez == -1 ? zp : z);
-        const uint8_t fs = flag[((long long)zs * g.ny + ys) * g.pitch + xs];
-        if (fs != 0) nonfluid_src = true;
-        if (fs == SW_WALL) wall_src = true;
+// Mirrors the pull-source mapping of the step (lbm3d.py:77-88).  One thread per
+// segment: the nine source rows' 32 flags each become two bit masks, shifted
+// along x for the sources at x - 1 and x + 1, so a segment takes 18 16-byte
+// loads instead of 19 byte loads per cell: 640x128x128, 506 -> 13 us.
+template <bool ALIGNED>
+__global__ void __launch_bounds__(256) k_build_tiles(Geom g, const uint8_t *flag, uint8_t *tiles) {
+  const uint32_t nseg = (uint32_t)(g.plane / SEG);
+  const uint32_t seg = blockIdx.x * 256u + threadIdx.x;
+  if (seg >= nseg) return;
+  const uint32_t row = seg / (uint32_t)g.nseg_x;
+  const int sx = (int)(seg - row * (uint32_t)g.nseg_x);
+  const int z = (int)(row / (uint32_t)g.ny), y = (int)(row - (uint32_t)z * (uint32_t)g.ny);
+  const int x0 = sx * SEG, left = g.nx - x0;                          // cells of the row from here on
+  const uint32_t live = left >= SEG ? 0xffffffffu : (1u << left) - 1u;
+  const int ys[3] = {y == 0 ? g.ny - 1 : y - 1, y, y == g.ny - 1 ? 0 : y + 1};
+  const int zs[3] = {z - 1, z, z == g.nz - 1 ? z : z + 1};            // the top copies its own level
+  uint32_t solid = 0u, wall = 0u, own = 0u;                           // sources of each cell, ORed
+#pragma unroll
+  for (int dz = 0; dz < 3; ++dz) {
+    if (zs[dz] < 0) {                                                 // below the bottom plane: ground
+      solid = 0xffffffffu;
+      continue;
+    }
+#pragma unroll
+    for (int dy = 0; dy < 3; ++dy) {
+      const uint8_t *p = flag + (((size_t)zs[dz] * g.ny + ys[dy]) * g.pitch + x0);
+      const SegMask m = seg_mask<ALIGNED>(p);
+      if (dz == 1 && dy == 1) own = m.solid;
+      else solid |= m.solid, wall |= m.wall;                          // the source at x
+      if (dz == 1 || dy == 1) {                                       // sources at x - 1 and x + 1
+        const uint8_t before = x0 > 0 ? p[-1] : (uint8_t)0;           // (the inlet does not pull)
+        const uint8_t after = left > SEG ? p[SEG] : (uint8_t)0;
+        uint32_t sn = (m.solid >> 1) | (after != 0 ? 0x80000000u : 0u), wn = (m.wall >> 1) | (after == SW_WALL ? 0x80000000u : 0u);
+        if (left <= SEG) {                                            // the outlet copies column nx - 1
+          const uint32_t last = 1u << (left - 1);
+          sn = (sn & ~last) | (m.solid & last);
+          wn = (wn & ~last) | (m.wall & last);
+        }
+        solid |= sn | (m.solid << 1) | (before != 0 ? 1u : 0u);
+        wall |= wn | (m.wall << 1) | (before == SW_WALL ? 1u : 0u);
       }
     }
   }
-  const unsigned any_fluid = __ballot_sync(0xffffffffu, live && fluid);
-  const unsigned any_check = __ballot_sync(0xffffffffu, live && (!fluid || nonfluid_src));
-  const unsigned any_wall = __ballot_sync(0xffffffffu, live && fluid && wall_src);
-  if (lane == 0)
-    tiles[seg] = (uint8_t)((any_fluid ? 0 : TILE_ALL_SOLID) | (any_check ? TILE_CHECK : 0) |
-                           (any_wall ? TILE_FORCE : 0));
+  const uint32_t fluid = live & ~own;
+  const uint32_t pulls = x0 == 0 ? fluid & ~1u : fluid;               // inlet cells do not pull
+  tiles[seg] = (uint8_t)((fluid ? 0 : TILE_ALL_SOLID) | ((live & own) | (pulls & solid) ? TILE_CHECK : 0) |
+                         (pulls & wall ? TILE_FORCE : 0));
 }
 
 // ---------------------------------------------------------------- x <-> z transposes
@@ -248,8 +340,9 @@ cudaError_t unpack_f_t(const Geom &g, int ref_dtype, const void *f, void *ref, c
 template <int DT>
 cudaError_t init_t(const Geom &g, void *f, const uint8_t *flag, const float *uin, float noise, int seed, int kind,
                    cudaStream_t s) {
-  const long long blocks = (g.plane + 255) / 256;
-  k_init<DT><<<(unsigned)blocks, 256, 0, s>>>(g, (typename Store<DT>::T *)f, flag, uin, noise, seed, kind);
+  constexpr int CPT = sizeof(typename Store<DT>::T) == 2 ? 2 : 1;
+  const long long blocks = (g.plane / CPT + 255) / 256;
+  k_init<DT, CPT><<<(unsigned)blocks, 256, 0, s>>>(g, (typename Store<DT>::T *)f, flag, uin, noise, seed, kind);
   return cudaGetLastError();
 }
 template <int DT>
@@ -300,8 +393,9 @@ cudaError_t aux_unpack_acc(const Geom &g, const double *acc, double *ref, cudaSt
   return cudaGetLastError();
 }
 cudaError_t aux_build_tiles(const Geom &g, const uint8_t *flag, uint8_t *tiles, cudaStream_t s) {
-  const long long blocks = (g.plane + 255) / 256;
-  k_build_tiles<<<(unsigned)blocks, 256, 0, s>>>(g, flag, tiles);
+  const unsigned blocks = (unsigned)((g.plane / SEG + 255) / 256);
+  if (((uintptr_t)flag & 15u) == 0) k_build_tiles<true><<<blocks, 256, 0, s>>>(g, flag, tiles);
+  else k_build_tiles<false><<<blocks, 256, 0, s>>>(g, flag, tiles);     // rows start on 32-byte offsets of it
   return cudaGetLastError();
 }
 
