@@ -4,6 +4,8 @@
 // (or every few steps) and evaluate every expression in source order, so their
 // float32 results equal the reference's operation sequence exactly (k_init for
 // the same random stream, k_macro for the same f).
+#include <cooperative_groups.h>
+
 #include "sw_aux.cuh"
 
 namespace sw {
@@ -413,109 +415,174 @@ cudaError_t aux_force_to_f64(const long long *fx, double *out, long long n, cuda
 // lbm3d.py:396-407: per step t, Fx = sum_z F_x(z), Fz = sum_z F_z(z) and the
 // overturning moment M = sum_z F_x(z) (z - 1/2) about the wall base, as
 // Cd = Fx / (q A), Cl = Fz / (q A), Cm = M / (q A H), q A = U_H^2 / 2 * H ny.
-// One warp per step: lanes over the levels (coalesced 16-byte rows), float64
-// partial sums combined by an xor butterfly in a fixed order.
-__global__ void k_coefficients(const long long *force, long long n_steps, int nz, double qa, double H,
-                               double *coef) {
-  const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (t >= n_steps) return;                                  // uniform across the warp
-  const longlong2 *row = reinterpret_cast<const longlong2 *>(force + t * 2 * nz);
-  double fx = 0.0, fz = 0.0, m = 0.0;
-  for (int z = lane; z < nz; z += 32) {
-    const longlong2 v = row[z];
-    const double x = (double)v.x * (1.0 / FORCE_SCALE), y = (double)v.y * (1.0 / FORCE_SCALE);
-    fx += x;
-    fz += y;
-    m += x * ((double)z - 0.5);
+// Eight lanes per step (a row of 16-byte levels is read 128 bytes at a time).
+// The sums over the levels are exact: the halves of the fixed-point values are
+// added as 64-bit integers and become doubles once per lane, because the FP64
+// pipe retires two operations per clock and SM, conversions included (nine of
+// them per level bounded the first form: 20 000 x 128 levels 100 us, now
+// 20 us).  kCoefLevels levels at a time keep the integer sums below 2^62.
+constexpr int kCoefLevels = 1 << 16;
+__global__ void __launch_bounds__(256) k_coefficients(const long long *force, long long n_steps, int nz, double qa,
+                                                      double H, double *coef) {
+  const long long t = ((long long)blockIdx.x * 256 + threadIdx.x) >> 3;
+  const int lane = threadIdx.x & 7;
+  double sum[3] = {0.0, 0.0, 0.0};                           // Fx, Fz, 2 M (in units of 1 / FORCE_SCALE)
+  if (t < n_steps) {
+    const longlong2 *row = reinterpret_cast<const longlong2 *>(force) + t * nz;
+    for (int z0 = 0; z0 < nz; z0 += kCoefLevels) {
+      const int n = nz - z0 < kCoefLevels ? nz - z0 : kCoefLevels;
+      long long xh = 0, xl = 0, zh = 0, zl = 0, mh = 0, ml = 0;
+#pragma unroll 4
+      for (int z = lane; z < n; z += 8) {
+        const longlong2 v = __ldg(row + z0 + z);
+        const int h = (int)(v.x >> 32), w = 2 * z - 1;
+        const uint32_t l = (uint32_t)v.x;
+        xh += h;
+        xl += l;
+        zh += (int)(v.y >> 32);
+        zl += (uint32_t)v.y;
+        mh += (long long)h * w;
+        ml += (long long)l * w;
+      }
+      const double fx = __fma_rn((double)xh, 4294967296.0, (double)xl);
+      sum[0] += fx;
+      sum[1] += __fma_rn((double)zh, 4294967296.0, (double)zl);
+      sum[2] += __fma_rn((double)mh, 4294967296.0, (double)ml);
+      if (z0 > 0) sum[2] += 2.0 * (double)z0 * fx;           // (uniform: rows this long are rare)
+    }
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    fx += __shfl_xor_sync(0xffffffffu, fx, o);
-    fz += __shfl_xor_sync(0xffffffffu, fz, o);
-    m += __shfl_xor_sync(0xffffffffu, m, o);
+  for (int o = 4; o > 0; o >>= 1) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
   }
-  if (lane == 0) {
-    coef[t] = fx / qa;
-    coef[n_steps + t] = fz / qa;
-    coef[2 * n_steps + t] = m / (qa * H);
-  }
+  // lane k writes coefficient k: Cd, Cl, Cm (one division per warp)
+  const double scale = lane == 2 ? 0.5 / FORCE_SCALE : 1.0 / FORCE_SCALE;
+  const double den = lane == 2 ? qa * H : qa, num = lane == 0 ? sum[0] : lane == 1 ? sum[1] : sum[2];
+  if (t < n_steps && lane < 3) coef[lane * n_steps + t] = num * scale / den;
 }
 
 // postprocess.py:65-82 over the steps t >= n_spin of the coefficient series:
 // stats = mean Cd, max Cd, std Cd (about the mean, two passes), mean Cm, max Cm,
-// mean Cl; NaN when no step is left.  One block; fixed reduction order.
-constexpr int kStatThreads = 512;
+// mean Cl; NaN when no step is left.  One cluster of blocks, partial results
+// exchanged through distributed shared memory, fixed reduction order.  Bound by
+// one SM's FP64 pipe as a single block (62 us for 20 000 steps, 16 us with
+// eight); the maxima compare bit patterns as integers for the same reason.
+constexpr int kStatThreads = 256, kStatBlocks = 8;
+struct StatPart {
+  double cd, cm, cl, dev;
+  long long max_cd, max_cm;
+};
+// doubles in the order of their values as signed integers; NaN as -infinity,
+// which a maximum starts from
+constexpr long long ordered_floor = (long long)0x800fffffffffffffull;
+__device__ __forceinline__ long long ordered(double v) {
+  const long long b = __double_as_longlong(v);
+  const long long k = b ^ ((b >> 63) & 0x7fffffffffffffffll);
+  return (b & 0x7fffffffffffffffll) > 0x7ff0000000000000ll ? ordered_floor : k;
+}
+__device__ __forceinline__ double unordered(long long k) {
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
+}
+// warp sums of this block in sh, added in warp order by every thread
 __device__ __forceinline__ double block_sum(double v, double *sh) {
-  const int tid = threadIdx.x;
-  sh[tid] = v;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
   __syncthreads();
-  for (int s = kStatThreads / 2; s > 0; s >>= 1) {
-    if (tid < s) sh[tid] += sh[tid + s];
-    __syncthreads();
-  }
-  const double r = sh[0];
+  if (threadIdx.x == 0)
+    for (int w = 1; w < kStatThreads / 32; ++w) v += sh[w];
   __syncthreads();
-  return r;
+  return v;                                                  // thread 0's is the block's
 }
-__device__ __forceinline__ double block_max(double v, double *sh) {
-  const int tid = threadIdx.x;
-  sh[tid] = v;
-  __syncthreads();
-  for (int s = kStatThreads / 2; s > 0; s >>= 1) {
-    if (tid < s) sh[tid] = fmax(sh[tid], sh[tid + s]);
-    __syncthreads();
+__device__ __forceinline__ long long block_max(long long v, long long *sh) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const long long w = __shfl_xor_sync(0xffffffffu, v, o);
+    v = w > v ? w : v;
   }
-  const double r = sh[0];
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
   __syncthreads();
-  return r;
+  if (threadIdx.x == 0)
+    for (int w = 1; w < kStatThreads / 32; ++w) v = sh[w] > v ? sh[w] : v;
+  __syncthreads();
+  return v;
 }
-__global__ void __launch_bounds__(kStatThreads) k_coef_stats(const double *coef, long long n_steps, long long n_spin,
-                                                            double *stats) {
-  __shared__ double sh[kStatThreads];
+__global__ void __cluster_dims__(kStatBlocks) __launch_bounds__(kStatThreads)
+    k_coef_stats(const double *coef, long long n_steps, long long n_spin, double *stats) {
+  namespace cg = cooperative_groups;
+  __shared__ StatPart part;
+  __shared__ double sh[kStatThreads / 32];
+  __shared__ long long shk[kStatThreads / 32];
+  cg::cluster_group cluster = cg::this_cluster();
   const double *cd = coef, *cl = coef + n_steps, *cm = coef + 2 * n_steps;
   const long long n = n_steps - n_spin;
-  if (n <= 0) {
-    if (threadIdx.x < 6) stats[threadIdx.x] = __longlong_as_double(0x7ff8000000000000ll);   // quiet NaN
+  if (n <= 0) {                                              // the same in every block
+    if (blockIdx.x == 0 && threadIdx.x < 6) stats[threadIdx.x] = __longlong_as_double(0x7ff8000000000000ll);
     return;
   }
-  double s_cd = 0.0, s_cm = 0.0, s_cl = 0.0, m_cd = -1.0 / 0.0, m_cm = -1.0 / 0.0;
-  for (long long t = n_spin + threadIdx.x; t < n_steps; t += kStatThreads) {
-    s_cd += cd[t];
-    s_cm += cm[t];
+  const long long first = n_spin + (long long)blockIdx.x * kStatThreads + threadIdx.x;
+  constexpr long long stride = (long long)kStatBlocks * kStatThreads;
+  double s_cd = 0.0, s_cm = 0.0, s_cl = 0.0;
+  long long m_cd = ordered_floor, m_cm = ordered_floor;
+#pragma unroll 4
+  for (long long t = first; t < n_steps; t += stride) {
+    const double a = cd[t], b = cm[t];
+    s_cd += a;
+    s_cm += b;
     s_cl += cl[t];
-    m_cd = fmax(m_cd, cd[t]);
-    m_cm = fmax(m_cm, cm[t]);
+    const long long ka = ordered(a), kb = ordered(b);
+    m_cd = ka > m_cd ? ka : m_cd;
+    m_cm = kb > m_cm ? kb : m_cm;
   }
-  const double mean_cd = block_sum(s_cd, sh) / (double)n;
-  const double mean_cm = block_sum(s_cm, sh) / (double)n;
-  const double mean_cl = block_sum(s_cl, sh) / (double)n;
-  const double max_cd = block_max(m_cd, sh), max_cm = block_max(m_cm, sh);
+  s_cd = block_sum(s_cd, sh);
+  s_cm = block_sum(s_cm, sh);
+  s_cl = block_sum(s_cl, sh);
+  m_cd = block_max(m_cd, shk);
+  m_cm = block_max(m_cm, shk);
+  if (threadIdx.x == 0) part = {s_cd, s_cm, s_cl, 0.0, m_cd, m_cm};
+  cluster.sync();
+  double mean_cd = 0.0;
+  for (int r = 0; r < kStatBlocks; ++r) mean_cd += cluster.map_shared_rank(&part, r)->cd;
+  mean_cd = mean_cd / (double)n;
   double s_dev = 0.0;
-  for (long long t = n_spin + threadIdx.x; t < n_steps; t += kStatThreads) {
+#pragma unroll 4
+  for (long long t = first; t < n_steps; t += stride) {
     const double d = cd[t] - mean_cd;
     s_dev += d * d;
   }
-  const double var = block_sum(s_dev, sh) / (double)n;
-  if (threadIdx.x == 0) {
+  s_dev = block_sum(s_dev, sh);
+  if (threadIdx.x == 0) part.dev = s_dev;
+  cluster.sync();
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    StatPart all = part;
+    for (int r = 1; r < kStatBlocks; ++r) {
+      const StatPart *o = cluster.map_shared_rank(&part, r);
+      all.cm += o->cm;
+      all.cl += o->cl;
+      all.dev += o->dev;
+      all.max_cd = o->max_cd > all.max_cd ? o->max_cd : all.max_cd;
+      all.max_cm = o->max_cm > all.max_cm ? o->max_cm : all.max_cm;
+    }
     stats[0] = mean_cd;
-    stats[1] = max_cd;
-    stats[2] = sqrt(var);
-    stats[3] = mean_cm;
-    stats[4] = max_cm;
-    stats[5] = mean_cl;
+    stats[1] = unordered(all.max_cd);
+    stats[2] = sqrt(all.dev / (double)n);
+    stats[3] = all.cm / (double)n;
+    stats[4] = unordered(all.max_cm);
+    stats[5] = all.cl / (double)n;
   }
+  cluster.sync();                                            // the other blocks' shared memory until read
 }
 
 cudaError_t aux_coefficients(const long long *force, long long n_steps, int nz, double qa, double H, double *coef,
                              cudaStream_t s) {
   if (n_steps <= 0) return cudaSuccess;
-  const long long threads = n_steps * 32;
+  const long long threads = n_steps * 8;
   k_coefficients<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(force, n_steps, nz, qa, H, coef);
   return cudaGetLastError();
 }
 cudaError_t aux_coef_stats(const double *coef, long long n_steps, long long n_spin, double *stats, cudaStream_t s) {
-  k_coef_stats<<<1, kStatThreads, 0, s>>>(coef, n_steps, n_spin, stats);
+  k_coef_stats<<<kStatBlocks, kStatThreads, 0, s>>>(coef, n_steps, n_spin, stats);
   return cudaGetLastError();
 }
 
