@@ -382,6 +382,17 @@ int sw_slice_xy(const sw_geom *g, const float *u, int32_t z0, float *out, sw_str
 int sw_qcoarse(const sw_geom *g, const float *u, const uint8_t *flag, int32_t x0, int32_t ds, int32_t di,
                int32_t dj, int32_t dk, float *out, sw_stream s);
 
+/* The planes of a snapshot as lbm3d.py:371-375 keeps them: ux, uy, uz of u at
+ * y = y0 as [3][nx][nz] and, behind them, at z = z0 as [3][nx][ny], in half
+ * precision (rounded to nearest; out: 3 nx (nz + ny) values, device). */
+int sw_snapshot_planes(const sw_geom *g, const float *u, int32_t y0, int32_t z0, void *out, sw_stream s);
+/* The quantisation of a Q frame to bytes (lbm3d.py:317-318) given its level
+ * boundaries: out[e] = how many of levels[0..255) (ascending) are at most
+ * min(q[e] * scale, qmax).  The host makes the levels with its own logarithm
+ * (stonewall/solver.py), so the bytes are the host expression's. */
+int sw_quantise_levels(const float *q, int64_t n, float scale, float qmax, const float *levels, uint8_t *out,
+                       sw_stream s);
+
 /* ---------------------------------------------------------------- step without allocation
  * No counterpart in the reference: an addition for callers that cannot
  * allocate device memory -- a host that only receives device pointers from an

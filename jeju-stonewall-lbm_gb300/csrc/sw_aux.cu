@@ -688,20 +688,65 @@ __device__ float q_at(const Geom &g, const float *u, const uint8_t *flag, int x,
 }
 
 // k_qcoarse (lbm3d.py:225-238): max of max(Q, 0) over ds^3 blocks of the crop
-// starting at (x0, 0, 0); out[i][j][k], one thread per output voxel.
-__global__ void k_qcoarse(Geom g, const float *u, const uint8_t *flag, int x0, int ds, int di, int dj, int dk,
-                          float *out) {
-  const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= (long long)di * dj * dk) return;
-  const int k = (int)(n % dk), j = (int)((n / dk) % dj), i = (int)(n / ((long long)dk * dj));
-  float best = 0.0f;
-  for (int a = 0; a < ds; ++a)
-    for (int b = 0; b < ds; ++b)
+// starting at (x0, 0, 0).  A block of threads takes `nb` neighbouring output
+// voxels of one (j, k): its threads run along x over their nb * ds cells, so the
+// 25 loads of a cell are coalesced (one thread per voxel, with neighbouring
+// threads ds levels apart, took 597 us for the 120x53x33 frame of an
+// 800x160x321 grid; this takes 72 us), and the maxima of a voxel meet in
+// shared memory as integers (they are not negative).
+constexpr int kQThreads = 128;
+__global__ void __launch_bounds__(kQThreads) k_qcoarse(Geom g, const float *u, const uint8_t *flag, int x0, int ds,
+                                                       int di, int dj, int dk, int nb, float *out) {
+  __shared__ int best[kQThreads];
+  const unsigned nbx = (unsigned)((di + nb - 1) / nb), jk = blockIdx.x / nbx;
+  const int i0 = (int)(blockIdx.x - jk * nbx) * nb;
+  const int j = (int)(jk / (unsigned)dk), k = (int)(jk - (unsigned)j * dk);
+  const int n = min(nb, di - i0);                            // voxels here (nb <= kQThreads)
+  if ((int)threadIdx.x < n) best[threadIdx.x] = 0;
+  __syncthreads();
+  for (int t = threadIdx.x; t < n * ds; t += kQThreads) {
+    const int x = x0 + i0 * ds + t;
+    float m = 0.0f;
+    if (x >= 1 && x < g.nx - 1)
       for (int c = 0; c < ds; ++c) {
-        const int x = x0 + i * ds + a, y = j * ds + b, z = k * ds + c;
-        if (x >= 1 && x < g.nx - 1 && z >= 1 && z < g.nz - 1) best = fmaxf(best, q_at(g, u, flag, x, y, z));
+        const int z = k * ds + c;
+        if (z < 1 || z >= g.nz - 1) continue;
+        for (int b = 0; b < ds; ++b) m = fmaxf(m, q_at(g, u, flag, x, j * ds + b, z));
       }
-  out[n] = best;
+    if (m > 0.0f) atomicMax(&best[t / ds], __float_as_int(m));
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < n) out[((long long)(i0 + (int)threadIdx.x) * dj + j) * dk + k] = __int_as_float(best[threadIdx.x]);
+}
+
+// The planes of a snapshot (lbm3d.py:371-375): ux, uy, uz at y = y0 as
+// [3][nx][nz], then at z = z0 as [3][nx][ny], rounded to half precision.
+__global__ void k_snapshot(Geom g, const float *u, int y0, int z0, __half *out) {
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long xz = 3ll * g.nx * g.nz, xy = 3ll * g.nx * g.ny;
+  if (e >= xz + xy) return;
+  const bool side = e < xz;
+  const uint32_t r = (uint32_t)(side ? e : e - xz), n = (uint32_t)(side ? g.nz : g.ny);
+  const uint32_t cx = r / n, w = r - cx * n, c = cx / (uint32_t)g.nx, x = cx - c * (uint32_t)g.nx;
+  const size_t row = side ? (size_t)w * g.ny + y0 : (size_t)z0 * g.ny + w;
+  out[e] = __float2half_rn(u[(size_t)(c + 1) * g.plane + row * g.pitch + x]);
+}
+
+// The log quantisation of a Q frame (lbm3d.py:317-318) by its level boundaries:
+// out = how many of the 255 ascending levels are <= min(q * scale, qmax).
+__global__ void __launch_bounds__(256) k_quantise(const float *q, long long n, float scale, float qmax,
+                                                  const float *levels, uint8_t *out) {
+  __shared__ float lev[256];
+  lev[threadIdx.x] = threadIdx.x < 255 ? levels[threadIdx.x] : __int_as_float(0x7f800000);
+  __syncthreads();
+  const long long e = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (e >= n) return;
+  const float v = fminf(__fmul_rn(q[e], scale), qmax);
+  int lo = 0;                                                // levels[0..lo) <= v
+#pragma unroll
+  for (int step = 128; step > 0; step >>= 1)
+    if (lev[lo + step - 1] <= v) lo += step;
+  out[e] = (uint8_t)lo;
 }
 
 cudaError_t aux_slice_xz(const Geom &g, const float *u, int y0, float *out, cudaStream_t s) {
@@ -716,9 +761,21 @@ cudaError_t aux_slice_xy(const Geom &g, const float *u, int z0, float *out, cuda
 }
 cudaError_t aux_qcoarse(const Geom &g, const float *u, const uint8_t *flag, int x0, int ds, int di, int dj, int dk,
                         float *out, cudaStream_t s) {
-  const long long n = (long long)di * dj * dk;
-  if (n == 0) return cudaSuccess;
-  k_qcoarse<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(g, u, flag, x0, ds, di, dj, dk, out);
+  if ((long long)di * dj * dk == 0) return cudaSuccess;
+  const int nb = ds < kQThreads ? kQThreads / ds : 1;        // as many voxels as a block has cells for
+  const long long blocks = (long long)((di + nb - 1) / nb) * dj * dk;
+  k_qcoarse<<<(unsigned)blocks, kQThreads, 0, s>>>(g, u, flag, x0, ds, di, dj, dk, nb, out);
+  return cudaGetLastError();
+}
+cudaError_t aux_snapshot(const Geom &g, const float *u, int y0, int z0, void *out, cudaStream_t s) {
+  const long long n = 3ll * g.nx * ((long long)g.nz + g.ny);
+  k_snapshot<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(g, u, y0, z0, static_cast<__half *>(out));
+  return cudaGetLastError();
+}
+cudaError_t aux_quantise(const float *q, long long n, float scale, float qmax, const float *levels, uint8_t *out,
+                         cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  k_quantise<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(q, n, scale, qmax, levels, out);
   return cudaGetLastError();
 }
 

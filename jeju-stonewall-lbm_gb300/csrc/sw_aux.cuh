@@ -28,6 +28,10 @@ cudaError_t aux_slice_xy(const Geom &g, const float *u, int z0, float *out, cuda
 cudaError_t aux_qcoarse(const Geom &g, const float *u, const uint8_t *flag, int x0, int ds, int di, int dj, int dk,
                         float *out, cudaStream_t s);
 
+cudaError_t aux_snapshot(const Geom &g, const float *u, int y0, int z0, void *out, cudaStream_t s);
+cudaError_t aux_quantise(const float *q, long long n, float scale, float qmax, const float *levels, uint8_t *out,
+                         cudaStream_t s);
+
 int note_cuda_error(int cuda_error);  // sw_capi.cu
 // largest wall box (bytes of its bitset) the ellipsoid packer holds in shared memory
 constexpr long long kPackBoxBytesMax = 200 * 1024;

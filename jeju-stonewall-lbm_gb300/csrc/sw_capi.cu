@@ -471,4 +471,18 @@ int sw_qcoarse(const sw_geom *g, const float *u, const uint8_t *flag, int32_t x0
   return cuda_status(sw::aux_qcoarse(to_geom(g), u, flag, x0, ds, di, dj, dk, out, st(s)));
 }
 
+int sw_snapshot_planes(const sw_geom *g, const float *u, int32_t y0, int32_t z0, void *out, sw_stream s) {
+  if (!geom_ok(g) || !u || !out || y0 < 0 || y0 >= g->ny || z0 < 0 || z0 >= g->nz) return SW_ERR_BAD_ARG;
+  if (((uintptr_t)out & 1u) || 3ll * g->nx * std::max(g->ny, g->nz) >= (1ll << 32)) return SW_ERR_BAD_ARG;
+  clear_stale();
+  return cuda_status(sw::aux_snapshot(to_geom(g), u, y0, z0, out, st(s)));
+}
+
+int sw_quantise_levels(const float *q, int64_t n, float scale, float qmax, const float *levels, uint8_t *out,
+                       sw_stream s) {
+  if (n < 0 || (n > 0 && (!q || !out)) || !levels) return SW_ERR_BAD_ARG;
+  clear_stale();
+  return cuda_status(sw::aux_quantise(q, n, scale, qmax, levels, out, st(s)));
+}
+
 }  // extern "C"

@@ -124,6 +124,8 @@ def load(path):
         "sw_pack_ellipsoids": ([P, i32, i32, i32, i32, i32, f64, P, P, P], ctypes.c_int),
         "sw_voxelize_stones": ([P, i32, i32, i32, i32, P, P, i32, P], ctypes.c_int),
         "sw_tma_timeouts": ([], i64),
+        "sw_snapshot_planes": ([G, P, i32, i32, P, P], ctypes.c_int),
+        "sw_quantise_levels": ([P, i64, f32, f32, P, P, P], ctypes.c_int),
         "sw_slice_xz": ([G, P, i32, P, P], ctypes.c_int),
         "sw_slice_xy": ([G, P, i32, P, P], ctypes.c_int),
         "sw_qcoarse": ([G, P, P, i32, i32, i32, i32, i32, P, P], ctypes.c_int),

@@ -16,6 +16,7 @@ in once complete.  force and uacc are stored in float64 (the reference writes
 float32), which makes a resumed run bit-identical to an uninterrupted one;
 float32 files from the reference load as well.
 """
+import functools
 import json
 import os
 import shutil
@@ -28,7 +29,7 @@ import torch
 from . import _native as N
 from . import kernels as K
 from . import trace
-from .fields import Accum, Flags, ForceSeries, Grid, Lattice, Macro, StatusWord
+from .fields import Accum, Flags, ForceSeries, Grid, Lattice, Macro, StatusWord, _ptr, _stream
 
 
 class Diverged(RuntimeError):
@@ -57,6 +58,27 @@ def status_exception(word, where):
     if err == N.SW_ERR_NONFINITE:
         return Diverged(f"{where}: non-finite density (status word {word:#x})")
     return None
+
+
+def _quantise(q, qmax):
+    """The reference's log quantisation of a clipped Q frame to bytes (lbm3d.py:317-318)."""
+    return np.round(255 * np.log1p(q) / np.log1p(qmax)).astype(np.uint8)
+
+
+@functools.lru_cache(maxsize=8)
+def quantise_levels(qmax):
+    """The smallest float32 that _quantise maps to k or more, for k = 1..255 (infinity if none up to
+    qmax is), found by bisection over the float32 values with _quantise itself: counting the levels
+    at or below a value gives its byte."""
+    top = int(np.float32(qmax).view(np.uint32))
+    k = np.arange(1, 256)
+    lo, hi = np.zeros(255, np.int64), np.full(255, top, np.int64)       # byte(lo) < k <= byte(hi)
+    while (hi - lo > 1).any():
+        mid = (lo + hi) // 2
+        up = _quantise(mid.astype(np.uint32).view(np.float32), qmax) >= k
+        lo, hi = np.where(up, lo, mid), np.where(up, mid, hi)
+    last = _quantise(np.array([top], np.uint32).view(np.float32), qmax)[0]
+    return np.where(k <= last, hi.astype(np.uint32).view(np.float32), np.float32(np.inf)).astype(np.float32)
 
 
 class WallSolver:
@@ -100,6 +122,7 @@ class WallSolver:
         self.n_acc = 0
         self.chunk = int(chunk)
         self._graphs = {}
+        self._q_levels = (None, None)   # quantisation levels of q_frame on the device, for one qmax
         self._ring = None
         self.launches = 0          # kernels of this library launched by advance()
         self._ckpt_host = None     # pinned host buffers of the checkpoint writer (reused)
@@ -279,11 +302,12 @@ class WallSolver:
         lbm3d.py:366-375 (k_macro, k_slice_xz, k_slice_xy, [1:].astype(float16))."""
         u = self._macro_dev()
         g = self.grid
-        xz = torch.empty((4, g.nx, g.nz), dtype=torch.float32, device=self.device)
-        xy = torch.empty((4, g.nx, g.ny), dtype=torch.float32, device=self.device)
-        K.k_slice_xz(u, y_mid, xz)
-        K.k_slice_xy(u, z_half, xy)
-        return xz.cpu().numpy()[1:].astype(np.float16), xy.cpu().numpy()[1:].astype(np.float16)
+        n = 3 * g.nx * g.nz
+        planes = torch.empty(n + 3 * g.nx * g.ny, dtype=torch.float16, device=self.device)
+        N.check(N.lib().sw_snapshot_planes(g.gp, u.ptr, int(y_mid), int(z_half), _ptr(planes), _stream(None)),
+                "sw_snapshot_planes")
+        host = planes.cpu().numpy()
+        return host[:n].reshape(3, g.nx, g.nz), host[n:].reshape(3, g.nx, g.ny)
 
     def q_frame(self, x0, ds, dims, q_scale, qmax=400.0, macro_ready=False):
         """Q-criterion frame of the current state: k_qcoarse then the reference's log quantisation
@@ -292,8 +316,17 @@ class WallSolver:
         q = torch.empty(tuple(dims), dtype=torch.float32, device=self.device)
         g = self.grid
         K.k_qcoarse(u, self.flags, x0, ds, g.nx, g.ny, g.nz, q)
-        q = np.clip(q.cpu().numpy() * q_scale, 0, qmax)
-        return np.round(255 * np.log1p(q) / np.log1p(qmax)).astype(np.uint8)
+        # q is float32, so plain numbers scale and clip it in float32; others (a numpy float64 would
+        # widen it) and limits without 255 levels below them stay with the expression itself
+        if type(q_scale) in (int, float) and type(qmax) in (int, float) and 0 < q_scale < 1e30 and 1e-3 < qmax < 1e30:
+            key = float(qmax)
+            if self._q_levels[0] != key:
+                self._q_levels = (key, torch.from_numpy(quantise_levels(key)).to(self.device))
+            out = torch.empty(tuple(dims), dtype=torch.uint8, device=self.device)
+            N.check(N.lib().sw_quantise_levels(_ptr(q), q.numel(), float(q_scale), key, _ptr(self._q_levels[1]),
+                                               _ptr(out), _stream(None)), "sw_quantise_levels")
+            return out.cpu().numpy()
+        return _quantise(np.clip(q.cpu().numpy() * q_scale, 0, qmax), qmax)
 
     def check_finite(self):
         if self.pattern == "aa" and not self.aa_odd_next:
@@ -328,8 +361,6 @@ class WallSolver:
         g = self.grid
         ref64 = self.dtype == 1
         main = torch.cuda.current_stream()
-        from . import _native as N
-        from .fields import _ptr, _stream
         f_dev = torch.empty((19, g.nx, g.ny, g.nz), dtype=torch.float64 if ref64 else torch.float32,
                             device=self.device)
         rd = N.SW_F64 if ref64 else N.SW_F32
