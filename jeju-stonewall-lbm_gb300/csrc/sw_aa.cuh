@@ -354,58 +354,39 @@ __device__ __forceinline__ void aa_pair_even_fast(const StepParams &p, int x0, i
 }
 
 // The collision and scatter of an interior odd-step cell pair (see
-// aa_pair_odd_interior), with the old float64 sums of the pair in acc_old.
-// inlet (lane 0 of the first segment pair, cell x0 = 0): that cell does not
-// pull (v holds its rest state) and scatters its inlet equilibrium
-// (lbm3d.py:67-71) instead of its collision, to the targets that exist and
-// are fluid (those in column 0 need not be: only cells of column 1 pull
-// from column 0).
-template <int DT, bool ACC>
-__device__ __forceinline__ void aa_pair_collide_scatter(const StepParams &p, const f2 (&v)[Q], int x0, int c, int z,
-                                                        int off_ym, int off_yp, int lev, int lane, bool inlet,
-                                                        const double2 (&acc_old)[4]) {
-  using S = Store<DT>;
-  using T = typename S::T;
+// aa_pair_odd_interior), with the old float64 sums of the pair in acc_old(k).
+// For c_x = +-1 the two targets lie in two aligned words: each is a 16-bit store.
+// (Words put together with the neighbouring lane by a shuffle, and 16-bit stores
+// by the first and last lane only, halve the stores but need predicates that
+// compile to branches: 640x128x128 without stones 184 us a step, 167 us like this.)
+template <int DT, bool ACC, typename AccOld>
+__device__ __forceinline__ void aa_pair_collide_scatter(const StepParams &p, const f2 (&v)[Q], int x0, int c, int off_ym,
+                                                        int off_yp, int lev, AccOld &&acc_old) {
+  using T = typename Store<DT>::T;
   using PK = Pack16<DT>;
   const Phys<float> ph = phys<float>(p);
-  const float u0 = inlet ? __ldg(p.uin + z) : 0.0f;
   f2 rho, ux, uy, uz;
   collide2(v, x0, true, ph.nu0, ph.c18, p.x_sponge, ph.sponge_scale, ph.nu_sponge, rho, ux, uy, uz, p.status,
            [&](auto I, f2 o) {
              constexpr int k = decltype(I)::value;
              constexpr int ex = CX(k), ey = CY(k), ez = CZ(k);
              T *plane = p.template out<T>(k);
-             const int t = c + (ey == 1 ? off_yp : ey == -1 ? off_ym : 0) + ez * lev;   // target row, column x0
-             if (inlet) {                                              // the inlet cell's equilibrium
-               float cu = 0.0f;
-               if constexpr (ex != 0) cu = (ex > 0 ? u0 : -u0);
-               cu = 3.0f * cu;
-               const float w = W<float>(k) * 1.0f * (1.0f + cu + 0.5f * cu * cu - 1.5f * (u0 * u0));
-               o.v.x = w - W<float>(k);
-             }
+             const int t = c + (ey == 1 ? off_yp : ey == -1 ? off_ym : 0) + ez * lev;
+             const uint32_t own = PK::pack(o.v.x, o.v.y);
              if constexpr (ex == 0) {
-               const int tw = chk(p, t);
-               if (!inlet || p.flag[tw] == 0) *reinterpret_cast<uint32_t *>(plane + tw) = PK::pack(o.v.x, o.v.y);
-               else plane[tw + 1] = S::from_shifted(o.v.y);            // column 0's target is not fluid
+               *reinterpret_cast<uint32_t *>(plane + chk(p, t)) = own;
              } else {
-               // targets x0 + ex (first cell) and x0 + 1 + ex (second cell); lane L writes the
-               // word holding its second target and lane L + 1's first
-               const float nxt = __shfl_down_sync(0xffffffffu, o.v.x, 1);
-               const int w = chk(p, t + (ex == 1 ? 2 : 0));
-               if (lane < 31) *reinterpret_cast<uint32_t *>(plane + w) = PK::pack(o.v.y, nxt);
-               else plane[w] = S::from_shifted(o.v.y);                 // the other half is the next warp's
-               if (lane == 0 && !(inlet && ex == -1))                  // the previous warp's (none left of the inlet)
-                 plane[chk(p, t + (ex == 1 ? 1 : -1))] = S::from_shifted(o.v.x);
+               uint16_t *half = reinterpret_cast<uint16_t *>(plane + chk(p, t));
+               half[ex] = (uint16_t)own;
+               half[ex + 1] = (uint16_t)(own >> 16);
              }
            });
   if (ACC) {
-    const double2 v0 = acc_old[0], v1 = acc_old[1], v2 = acc_old[2], v3 = acc_old[3];
-    const double ra = inlet ? 1.0 : (double)rho.v.x, xa = inlet ? (double)u0 : (double)ux.v.x;
-    const double ya = inlet ? 0.0 : (double)uy.v.x, za = inlet ? 0.0 : (double)uz.v.x;
-    *reinterpret_cast<double2 *>(p.accp(0) + c) = make_double2(v0.x + ra, v0.y + (double)rho.v.y);
-    *reinterpret_cast<double2 *>(p.accp(1) + c) = make_double2(v1.x + xa, v1.y + (double)ux.v.y);
-    *reinterpret_cast<double2 *>(p.accp(2) + c) = make_double2(v2.x + ya, v2.y + (double)uy.v.y);
-    *reinterpret_cast<double2 *>(p.accp(3) + c) = make_double2(v3.x + za, v3.y + (double)uz.v.y);
+    const double2 v0 = acc_old(0), v1 = acc_old(1), v2 = acc_old(2), v3 = acc_old(3);
+    *reinterpret_cast<double2 *>(p.accp(0) + c) = make_double2(v0.x + (double)rho.v.x, v0.y + (double)rho.v.y);
+    *reinterpret_cast<double2 *>(p.accp(1) + c) = make_double2(v1.x + (double)ux.v.x, v1.y + (double)ux.v.y);
+    *reinterpret_cast<double2 *>(p.accp(2) + c) = make_double2(v2.x + (double)uy.v.x, v2.y + (double)uy.v.y);
+    *reinterpret_cast<double2 *>(p.accp(3) + c) = make_double2(v3.x + (double)uz.v.x, v3.y + (double)uz.v.y);
   }
 }
 
@@ -413,9 +394,6 @@ __device__ __forceinline__ void aa_pair_collide_scatter(const StepParams &p, con
 // segment pair, not the top level; every pull source and scatter target is a
 // fluid cell inside the lattice): pull as the two-lattice pair kernel does, then
 // scatter S_k of both cells to slot k of x + c_k (fout_pop[k] = plane opp(k)).
-// For c_x = +-1 the two targets straddle two aligned words: lane L writes the
-// word that holds its second target and lane L + 1's first (one shuffle); the
-// halves at the warp's edges, shared with the neighbouring warps, are 16-bit stores.
 template <int DT, bool ACC>
 __device__ __forceinline__ void aa_pair_odd_interior(const StepParams &p, int x0, int y, int z, int lane) {
   using S = Store<DT>;
@@ -457,7 +435,7 @@ __device__ __forceinline__ void aa_pair_odd_interior(const StepParams &p, int x0
       v[i] = F2(own.y, lane == 31 ? edge[i] : PK::lo(next));
     }
   });
-  aa_pair_collide_scatter<DT, ACC>(p, v, x0, c, z, off_ym, off_yp, lev, lane, false, acc_old);
+  aa_pair_collide_scatter<DT, ACC>(p, v, x0, c, off_ym, off_yp, lev, [&](int k) { return acc_old[k]; });
 }
 
 // Grid: (ceil(pitch / 64), ceil(ny / WY), nz); warp = two adjacent row segments.
@@ -505,11 +483,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
 // The AA steps with their sources staged in shared memory by TMA, as k_step_tma
 // does for the two-lattice step (one item of 4 rows x 64 cells per block, all
 // copies issued at the start, bounded waits).  Odd step: the boxes are the
-// two-lattice step's (natural planes at the source rows and levels); a warp
-// not in the outlet segment pair, not at the top level and not next to stones
-// or the ground pulls from them and scatters as aa_pair_odd_interior does (the
-// inlet cell of the first pair scatters its equilibrium); the other warps run
-// the per-cell odd step.  Even step: box i is plane opp(i) -- slot i -- at
+// two-lattice step's (natural planes at the source rows and levels); interior
+// warps pull from them and scatter with aa_pair_collide_scatter, the others with
+// aa_odd_pair_edge.  Even step: box i is plane opp(i) -- slot i -- at
 // the item's own rows and level; every warp collides from it as
 // aa_pair_even_fast does, warps next to stones or the ground with the link
 // masks of their cells (the stone links' force, cells that are not fluid left
@@ -528,6 +504,235 @@ __device__ __forceinline__ void tma_issue_own(const CUtensorMap *map, const CUte
     tma_load_4d(st + i * kTmaBoxBytes, map, x0 - 8, y0, z, OPP(i), bar);
   });
   if constexpr (ACC) tma_load_4d(st + kTmaStageBytes, map_acc, x0, y0, z, 0, bar);
+}
+
+// The populations with c_x = -1 that the outlet cell of (y, z) pulls: column nx - 1 before the step (the ghost).
+template <int DT>
+__device__ __forceinline__ void aa_outlet_copies(const Geom &g, const AAParams &a, int y, int z, float (&copy)[kGhostPops]) {
+  using T = typename Store<DT>::T;
+  const T *ghost = static_cast<const T *>(a.ghost);
+  const size_t gp = (size_t)g.ny * g.nz;
+  const bool top = z == g.nz - 1;
+  static_for<0, Q>([&](auto I) {
+    constexpr int i = decltype(I)::value;
+    constexpr int ey = CY(i), ez = CZ(i), jm = MIRZ(i);
+    if constexpr (CX(i) == -1) {
+      const int ys = ey == 1 ? (y == 0 ? g.ny - 1 : y - 1) : ey == -1 ? (y == g.ny - 1 ? 0 : y + 1) : y;
+      const int zs = ez == 1 ? z - 1 : (ez == -1 ? (top ? z : z + 1) : z);
+      if (zs >= 0)                                                  // (the ground below z = 0 bounces)
+        copy[GIDX(i)] =
+            Store<DT>::template ld<i>(ghost + (ez == -1 && top ? GIDX(jm) : GIDX(i)) * gp + (size_t)zs * g.ny + ys);
+    }
+  });
+}
+
+// Odd step, the inlet or outlet segment pair or the top level, away from stones
+// and the ground, or a periodic edge row in y: pulled from the boxes like the
+// interior, the outlet copies from the ghost (`copy`), scattered by the rules at
+// the top of this file, one 16-bit store per target.  The inlet cell scatters its
+// equilibrium (lbm3d.py:67-71); its targets in column 0 need not be fluid.  The
+// outlet pair and the top level collide one cell at a time, in the operations of
+// aa_odd_cell, the others as the interior does.
+template <int DT, bool ACC>
+__device__ __forceinline__ void aa_odd_pair_edge(const StepParams &p, const uint8_t *smem, const float (&copy)[kGhostPops],
+                                              int x0, int y, int z, int w, int lane, bool outlet_pair) {
+  using T = typename Store<DT>::T;
+  using PK = Pack16<DT>;
+  const Geom &g = p.g;
+  const int row = g.pitch, lev = g.ny * g.pitch;
+  const int off_ym = (y == 0) ? (g.ny - 1) * row : -row;
+  const int off_yp = (y == g.ny - 1) ? -(g.ny - 1) * row : row;
+  const bool top = z == g.nz - 1, has_b = x0 + 1 < g.nx, has_r = x0 + 2 < g.nx;
+  const bool inlet = x0 == 0;
+  const int c = (z * g.ny + y) * g.pitch + x0;
+  const int lane_word = 4 + lane;
+  f2 v[Q];
+  static_for<0, Q>([&](auto I) {
+    constexpr int i = decltype(I)::value;
+    constexpr int ex = CX(i), ey = CY(i);
+    const uint8_t *rowp = smem + i * kTmaBoxBytes + w * kTmaRowBytes;
+    if constexpr (ey == 1) {
+      if (y == 0) rowp = smem + Q * kTmaBoxBytes + wrap_slot(i) * kTmaWrapBytes;
+    } else if constexpr (ey == -1) {
+      if (y == g.ny - 1) rowp = smem + Q * kTmaBoxBytes + wrap_slot(i) * kTmaWrapBytes;
+    }
+    const uint32_t *r = reinterpret_cast<const uint32_t *>(rowp);
+    const uint32_t own = r[lane_word];
+    if constexpr (ex == 0) {
+      v[i].v = PK::both(own);
+    } else if constexpr (ex == 1) {
+      v[i] = F2(PK::hi(r[lane_word - 1]), PK::lo(own));
+    } else {
+      v[i] = F2(has_b ? PK::hi(own) : copy[GIDX(i)], has_r ? PK::lo(r[lane_word + 1]) : copy[GIDX(i)]);
+    }
+    if (inlet) v[i].v.x = 0.0f;                                     // the inlet cell does not pull
+  });
+  if (x0 >= g.nx) return;
+  const float u0 = inlet ? __ldg(p.uin + z) : 0.0f;
+  auto put = [&](auto I, f2 o) {
+    constexpr int k = decltype(I)::value;
+    constexpr int ex = CX(k), ey = CY(k), ez = CZ(k);
+    T *plane = ez == 1 && top ? p.template out<T>(MIRZ(k)) : p.template out<T>(k);
+    const int t = c + (ey == 1 ? off_yp : ey == -1 ? off_ym : 0) + (ez == 1 && top ? 0 : ez * lev);
+    if (inlet) {
+      float cu = 0.0f;
+      if constexpr (ex != 0) cu = (ex > 0 ? u0 : -u0);
+      cu = 3.0f * cu;
+      const float e = W<float>(k) * 1.0f * (1.0f + cu + 0.5f * cu * cu - 1.5f * (u0 * u0));
+      o.v.x = e - W<float>(k);
+    }
+    const uint32_t own = PK::pack(o.v.x, o.v.y);
+    const int tw = chk(p, t);
+    uint16_t *half = reinterpret_cast<uint16_t *>(plane + tw);
+    if constexpr (ex == 0) {
+      if (inlet && p.flag[tw] != 0) half[1] = (uint16_t)(own >> 16);
+      else *reinterpret_cast<uint32_t *>(half) = own;                // (x0 + 1 may be padding)
+    } else {
+      if (ex == 1 ? has_b : !inlet) half[ex] = (uint16_t)own;
+      if (ex == 1 ? has_r : has_b) half[ex + 1] = (uint16_t)(own >> 16);
+      if constexpr (ex == -1) {                                     // (b): the outlet cell's own column
+        if (!has_r) half[has_b ? 1 : 0] = (uint16_t)(has_b ? own >> 16 : own);
+      }
+    }
+  };
+  const Phys<float> ph = phys<float>(p);
+  float m[2][4];                                                    // rho, u of both cells
+  if (outlet_pair || top) {
+    f2 o[Q];
+    float f[Q];
+    static_for<0, Q>([&](auto I) { f[decltype(I)::value] = v[decltype(I)::value].v.x; });
+    collide<float, true>(f, x0, ph.nu0, ph.c18, p.x_sponge, ph.sponge_scale, ph.nu_sponge, m[0][0], m[0][1], m[0][2],
+                         m[0][3], p.status, [&](auto I, float r) { o[decltype(I)::value].v.x = r; });
+    static_for<0, Q>([&](auto I) { f[decltype(I)::value] = v[decltype(I)::value].v.y; });
+    collide<float, true>(f, x0 + 1, ph.nu0, ph.c18, p.x_sponge, ph.sponge_scale, ph.nu_sponge, m[1][0], m[1][1],
+                         m[1][2], m[1][3], has_b ? p.status : nullptr,
+                         [&](auto I, float r) { o[decltype(I)::value].v.y = r; });
+    static_for<0, Q>([&](auto I) { put(I, o[decltype(I)::value]); });
+  } else {
+    f2 rho, ux, uy, uz;
+    collide2(v, x0, true, ph.nu0, ph.c18, p.x_sponge, ph.sponge_scale, ph.nu_sponge, rho, ux, uy, uz, p.status, put);
+    m[0][0] = rho.v.x, m[0][1] = ux.v.x, m[0][2] = uy.v.x, m[0][3] = uz.v.x;
+    m[1][0] = rho.v.y, m[1][1] = ux.v.y, m[1][2] = uy.v.y, m[1][3] = uz.v.y;
+  }
+  if (ACC) {
+    if (inlet) m[0][0] = 1.0f, m[0][1] = u0, m[0][2] = 0.0f, m[0][3] = 0.0f;
+    const double2 *acc_box = reinterpret_cast<const double2 *>(smem + kTmaStageBytes) + w * 32 + lane;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const double2 old = acc_box[k * 4 * 32];
+      p.accp(k)[c] = old.x + (double)m[0][k];
+      if (has_b) p.accp(k)[c + 1] = old.y + (double)m[1][k];
+    }
+  }
+}
+
+// The link masks and bounce-back pairs of a lane's cells (pair_links_prefetch).
+struct AALinks {
+  uint32_t sm[2], wm[2], bnc[Q];
+};
+
+// Odd step next to stones or the ground: as aa_odd_pair_edge, with the links and
+// bounce-back values that were fetched during the copies.  The target x + c_k of
+// rule (a), or of (c) at the top, is the pull source of opp(k), so the cell's link
+// mask says whether it is fluid; only the inlet cell, which does not pull, and the
+// outlet cell's second targets look at flags.  One cell at a time through
+// aa_odd_cell, these warps waited for 19 flag-dependent loads in a row: 4 % of the
+// segments of the 640x128x128 wall took 33 us of the step, and take 25 us here.
+template <int DT, bool ACC>
+__device__ __forceinline__ void aa_odd_pair_checked(const StepParams &p, const uint8_t *smem, const AALinks &f,
+                                                    const float (&copy)[kGhostPops], int x0, int y, int z, int w,
+                                                    int lane, bool force) {
+  using T = typename Store<DT>::T;
+  using PK = Pack16<DT>;
+  const Geom &g = p.g;
+  const int row = g.pitch, lev = g.ny * g.pitch;
+  const int off_ym = (y == 0) ? (g.ny - 1) * row : -row;
+  const int off_yp = (y == g.ny - 1) ? -(g.ny - 1) * row : row;
+  const bool top = z == g.nz - 1, has_b = x0 + 1 < g.nx, has_r = x0 + 2 < g.nx;
+  const int c = (z * g.ny + y) * g.pitch + x0;
+  const int lane_word = 4 + lane;
+  float fxw = 0.0f, fzw = 0.0f;
+  int hit = 0;
+  f2 v[Q];
+  static_for<0, Q>([&](auto I) {
+    constexpr int i = decltype(I)::value;
+    constexpr int ex = CX(i), ey = CY(i);
+    const uint8_t *rowp = smem + i * kTmaBoxBytes + w * kTmaRowBytes;
+    if constexpr (ey == 1) {
+      if (y == 0) rowp = smem + Q * kTmaBoxBytes + wrap_slot(i) * kTmaWrapBytes;
+    } else if constexpr (ey == -1) {
+      if (y == g.ny - 1) rowp = smem + Q * kTmaBoxBytes + wrap_slot(i) * kTmaWrapBytes;
+    }
+    const uint32_t *r = reinterpret_cast<const uint32_t *>(rowp);
+    const uint32_t own = r[lane_word];
+    if constexpr (ex == 0) {
+      v[i].v = PK::both(own);
+    } else if constexpr (ex == 1) {
+      v[i] = F2(PK::hi(r[lane_word - 1]), PK::lo(own));
+    } else {
+      v[i] = F2(has_b ? PK::hi(own) : copy[GIDX(i)], has_r ? PK::lo(r[lane_word + 1]) : copy[GIDX(i)]);
+    }
+    if constexpr (i > 0) pair_link<DT, i>(v[i], f.sm, f.wm, f.bnc[i], fxw, fzw, hit);
+    if (x0 == 0) v[i].v.x = 0.0f;                                   // the inlet cell does not pull
+  });
+  const uint32_t keep = pair_solid_cells(v, f.sm);
+  if (keep != 0u) {
+    const Phys<float> ph = phys<float>(p);
+    uint32_t o[Q];                                                  // the new populations, packed
+    float m[2][4];                                                  // rho, u of both cells
+    float in[Q];
+    static_for<0, Q>([&](auto I) { in[decltype(I)::value] = v[decltype(I)::value].v.x; });
+    collide<float, true>(in, x0, ph.nu0, ph.c18, p.x_sponge, ph.sponge_scale, ph.nu_sponge, m[0][0], m[0][1], m[0][2],
+                         m[0][3], p.status, [&](auto I, float r) { o[decltype(I)::value] = PK::pack(r, 0.0f); });
+    static_for<0, Q>([&](auto I) { in[decltype(I)::value] = v[decltype(I)::value].v.y; });
+    collide<float, true>(in, x0 + 1, ph.nu0, ph.c18, p.x_sponge, ph.sponge_scale, ph.nu_sponge, m[1][0], m[1][1],
+                         m[1][2], m[1][3], p.status,
+                         [&](auto I, float r) { o[decltype(I)::value] |= PK::pack(0.0f, r); });
+    const bool inlet = x0 == 0 && (keep & 1u);
+    const float u0 = inlet ? __ldg(p.uin + z) : 0.0f;
+    static_for<0, Q>([&](auto I) {
+      constexpr int k = decltype(I)::value;
+      constexpr int ex = CX(k), ey = CY(k), ez = CZ(k);
+      T *plane = ez == 1 && top ? p.template out<T>(MIRZ(k)) : p.template out<T>(k);
+      T *self = p.template out<T>(OPP(k));
+      const int t = c + (ey == 1 ? off_yp : ey == -1 ? off_ym : 0) + (ez == 1 && top ? 0 : ez * lev);
+      const bool below = ez == -1 && z == 0;                        // no such target
+      uint32_t val = o[k];
+      if (inlet) {
+        float cu = 0.0f;
+        if constexpr (ex != 0) cu = (ex > 0 ? u0 : -u0);
+        cu = 3.0f * cu;
+        const float e = W<float>(k) * 1.0f * (1.0f + cu + 0.5f * cu * cu - 1.5f * (u0 * u0));
+        val = (val & 0xffff0000u) | PK::pack(e - W<float>(k), 0.0f);
+      }
+      auto put = [&](T *at, int off, int h) {
+        *reinterpret_cast<uint16_t *>(at + chk(p, off)) = (uint16_t)(h ? val >> 16 : val);
+      };
+      auto fluid = [&](int off) { return p.flag[chk(p, off)] == 0; };
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (!((keep >> h) & 1u)) continue;
+        const bool in = h == 0 && inlet, last = h == 0 ? !has_b : !has_r;   // the inlet / outlet cell
+        if ((f.sm[h] >> OPP(k)) & 1u) {
+          put(self, c + h, h);                                      // (d)
+        } else if (!below && (ex != 1 || !last) && (ex != -1 || x0 + h > 0)) {
+          if (!in || fluid(t + h + ex)) put(plane, t + h + ex, h);   // (a), (c)
+        }
+        if (ex == -1 && last && !below && fluid(t + h)) put(plane, t + h, h);   // (b), (c)
+      }
+    });
+    if (ACC) {
+      if (inlet) m[0][0] = 1.0f, m[0][1] = u0, m[0][2] = 0.0f, m[0][3] = 0.0f;
+      const double2 *acc_box = reinterpret_cast<const double2 *>(smem + kTmaStageBytes) + w * 32 + lane;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const double2 old = acc_box[k * 4 * 32];
+        if (keep & 1u) p.accp(k)[c] = old.x + (double)m[0][k];
+        if (keep & 2u) p.accp(k)[c + 1] = old.y + (double)m[1][k];
+      }
+    }
+  }
+  if (force && p.force != nullptr) warp_force_add<float>(p, z, lane, fxw, fzw, hit);
 }
 
 template <int DT, bool ODD, bool ACC>
@@ -567,101 +772,95 @@ __global__ void __launch_bounds__(128, 9)
     cell_links(p, x0, y, z, sm[0], wm[0]);
     cell_links(p, x0 + 1, y, z, sm[1], wm[1]);
   }
+  const bool work = y < g.ny && !(ka & kb & TILE_ALL_SOLID);
+  // odd step off the interior path (uniform across the warp)
+  const bool checked = ((ka | kb) & TILE_CHECK) || z == 0;            // (a lone inlet column may be open at z = 0)
+  const bool outlet_pair = x0s + 2 * SEG >= g.nx;
+  const bool edge = !checked && (outlet_pair || x0s == 0 || z == g.nz - 1 || y == 0 || y == g.ny - 1);
+  AALinks links;
+  float copy[kGhostPops];
+  if (ODD && work && checked) {
+    links.sm[0] = links.sm[1] = 1u;
+    pair_links_prefetch<DT>(p, x0, y, z, links.sm, links.wm, links.bnc);
+  }
+  if (ODD && work && x0 <= g.nx - 1 && x0 + 1 >= g.nx - 1) aa_outlet_copies<DT>(g, a, y, z, copy);
   bool ok = mbar_wait(smem_u32(&bar), 0u, p.tma_poll_limit);
-  if (ok && y < g.ny && !(ka & kb & TILE_ALL_SOLID)) {
-    const int row = g.pitch, lev = g.ny * g.pitch;
+  if (ok && work) {
     const int lane_word = 4 + lane;                                   // 32-bit word of elements 8 + 2 lane, + 1
-    if (even_checked) {
-      // The even step reads the cell's own slots, where the odd step already put the
-      // bounce-back values (rule (d)); a link from a stone adds -2 (f - w) c of its
-      // value to the wall force (lbm3d.py:91-101), cell x0 before x0 + 1, as
-      // aa_even_cell adds them; cells that are not fluid are not stored.
-      float fxw = 0.0f, fzw = 0.0f;
-      int hit = 0;
-      if (x0 < g.nx) {
-        const bool has_b = x0 + 1 < g.nx;
-        const int c = chk(p, (z * g.ny + y) * g.pitch + x0);
-        f2 v[Q];
-        static_for<0, Q>([&](auto I) {
-          constexpr int i = decltype(I)::value;
-          v[i].v = PK::both(reinterpret_cast<const uint32_t *>(smem + i * kTmaBoxBytes + w * kTmaRowBytes)[lane_word]);
-        });
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          static_for<1, Q>([&](auto I) {
+    if constexpr (!ODD) {
+      if (even_checked) {
+        // The even step reads the cell's own slots, where the odd step already put the
+        // bounce-back values (rule (d)); a link from a stone adds -2 (f - w) c of its
+        // value to the wall force (lbm3d.py:91-101), cell x0 before x0 + 1, as
+        // aa_even_cell adds them; cells that are not fluid are not stored.
+        float fxw = 0.0f, fzw = 0.0f;
+        int hit = 0;
+        if (x0 < g.nx) {
+          const bool has_b = x0 + 1 < g.nx;
+          const int c = chk(p, (z * g.ny + y) * g.pitch + x0);
+          f2 v[Q];
+          static_for<0, Q>([&](auto I) {
             constexpr int i = decltype(I)::value;
-            constexpr int ex = CX(i), ez = CZ(i);
-            if ((wm[h] >> i) & 1u) {
-              const float fr = h ? v[i].v.y : v[i].v.x;
-              if constexpr (ex != 0) fxw = fxw - 2.0f * fr * (float)ex;
-              if constexpr (ez != 0) fzw = fzw - 2.0f * fr * (float)ez;
-              hit = 1;
-            }
+            v[i].v = PK::both(reinterpret_cast<const uint32_t *>(smem + i * kTmaBoxBytes + w * kTmaRowBytes)[lane_word]);
           });
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            static_for<1, Q>([&](auto I) {
+              constexpr int i = decltype(I)::value;
+              constexpr int ex = CX(i), ez = CZ(i);
+              if ((wm[h] >> i) & 1u) {
+                const float fr = h ? v[i].v.y : v[i].v.x;
+                if constexpr (ex != 0) fxw = fxw - 2.0f * fr * (float)ex;
+                if constexpr (ez != 0) fzw = fzw - 2.0f * fr * (float)ez;
+                hit = 1;
+              }
+            });
+          }
+          const uint32_t keep = pair_solid_cells(v, sm);
+          if (keep != 0u) {
+            const double2 *acc_box = reinterpret_cast<const double2 *>(smem + kTmaStageBytes) + w * 32 + lane;
+            pair_collide_store<DT, ACC, true>(p, v, x0, c, z, x0 == 0, has_b,
+                                              [&](int k) { return acc_box[k * 4 * 32]; }, keep);
+          }
         }
-        const uint32_t keep = pair_solid_cells(v, sm);
-        if (keep != 0u) {
+        if (((ka | kb) & TILE_FORCE) && p.force != nullptr) warp_force_add<float>(p, z, lane, fxw, fzw, hit);
+      } else {                                                          // even step: own slots, local
+        if (x0 < g.nx) {
+          const bool has_b = x0 + 1 < g.nx;
+          const int c = chk(p, (z * g.ny + y) * g.pitch + x0);
+          f2 v[Q];
+          static_for<0, Q>([&](auto I) {
+            constexpr int i = decltype(I)::value;
+            v[i].v = PK::both(reinterpret_cast<const uint32_t *>(smem + i * kTmaBoxBytes + w * kTmaRowBytes)[lane_word]);
+          });
           const double2 *acc_box = reinterpret_cast<const double2 *>(smem + kTmaStageBytes) + w * 32 + lane;
-          pair_collide_store<DT, ACC, true>(p, v, x0, c, z, x0 == 0, has_b,
-                                            [&](int k) { return acc_box[k * 4 * 32]; }, keep);
+          pair_collide_store<DT, ACC>(p, v, x0, c, z, x0 == 0, has_b, [&](int k) { return acc_box[k * 4 * 32]; });
         }
       }
-      if (((ka | kb) & TILE_FORCE) && p.force != nullptr) warp_force_add<float>(p, z, lane, fxw, fzw, hit);
-    } else if (!((ka | kb) & TILE_CHECK) && !ODD) {                   // even step: own slots, local
-      if (x0 < g.nx) {
-        const bool has_b = x0 + 1 < g.nx;
+    } else {
+      if (edge) {
+        aa_odd_pair_edge<DT, ACC>(p, smem, copy, x0, y, z, w, lane, outlet_pair);
+      } else if (checked) {                                           // odd step next to stones or the ground
+        aa_odd_pair_checked<DT, ACC>(p, smem, links, copy, x0, y, z, w, lane, (ka | kb) & TILE_FORCE);
+      } else {                                                        // odd step, interior
+        const int row = g.pitch, lev = g.ny * g.pitch;
         const int c = chk(p, (z * g.ny + y) * g.pitch + x0);
         f2 v[Q];
         static_for<0, Q>([&](auto I) {
           constexpr int i = decltype(I)::value;
-          v[i].v = PK::both(reinterpret_cast<const uint32_t *>(smem + i * kTmaBoxBytes + w * kTmaRowBytes)[lane_word]);
+          constexpr int ex = CX(i);
+          const uint32_t *r = reinterpret_cast<const uint32_t *>(smem + i * kTmaBoxBytes + w * kTmaRowBytes);
+          const uint32_t own = r[lane_word];                          // cells x0, x0 + 1
+          if constexpr (ex == 0) {
+            v[i].v = PK::both(own);
+          } else if constexpr (ex == 1) {                             // sources x0 - 1, x0
+            v[i] = F2(PK::hi(r[lane_word - 1]), PK::lo(own));
+          } else {                                                    // sources x0 + 1, x0 + 2
+            v[i] = F2(PK::hi(own), PK::lo(r[lane_word + 1]));
+          }
         });
         const double2 *acc_box = reinterpret_cast<const double2 *>(smem + kTmaStageBytes) + w * 32 + lane;
-        pair_collide_store<DT, ACC>(p, v, x0, c, z, x0 == 0, has_b, [&](int k) { return acc_box[k * 4 * 32]; });
-      }
-    } else if (!((ka | kb) & TILE_CHECK) && x0s + 2 * SEG < g.nx && z < g.nz - 1) {   // odd: not the outlet or top
-      const bool inlet = x0 == 0;                                     // lane 0 of the first pair
-      const int c = chk(p, (z * g.ny + y) * g.pitch + x0);
-      const int off_ym = (y == 0) ? (g.ny - 1) * row : -row;
-      const int off_yp = (y == g.ny - 1) ? -(g.ny - 1) * row : row;
-      f2 v[Q];
-      static_for<0, Q>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        constexpr int ex = CX(i), ey = CY(i);
-        const uint8_t *rowp = smem + i * kTmaBoxBytes + w * kTmaRowBytes;
-        if constexpr (ey == 1) {
-          if (y == 0) rowp = smem + Q * kTmaBoxBytes + wrap_slot(i) * kTmaWrapBytes;
-        } else if constexpr (ey == -1) {
-          if (y == g.ny - 1) rowp = smem + Q * kTmaBoxBytes + wrap_slot(i) * kTmaWrapBytes;
-        }
-        const uint32_t *r = reinterpret_cast<const uint32_t *>(rowp);
-        const uint32_t own = r[lane_word];                            // cells x0, x0 + 1
-        if constexpr (ex == 0) {
-          v[i].v = PK::both(own);
-        } else if constexpr (ex == 1) {                               // sources x0 - 1, x0
-          v[i] = F2(PK::hi(r[lane_word - 1]), PK::lo(own));
-        } else {                                                      // sources x0 + 1, x0 + 2
-          v[i] = F2(PK::hi(own), PK::lo(r[lane_word + 1]));
-        }
-        if (inlet) v[i].v.x = 0.0f;                                   // the inlet cell does not pull
-      });
-      double2 acc_old[4];
-      if (ACC) {
-        const double2 *acc_box = reinterpret_cast<const double2 *>(smem + kTmaStageBytes) + w * 32 + lane;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) acc_old[k] = acc_box[k * 4 * 32];
-      }
-      aa_pair_collide_scatter<DT, ACC>(p, v, x0, c, z, off_ym, off_yp, lev, lane, inlet, acc_old);
-    } else {                                                          // per cell (from the lattice)
-      float fxw = 0.0f, fzw = 0.0f;
-      int hit = 0;
-      if ((ka | kb) & TILE_CHECK) {                                   // odd step next to stones or the ground
-        if (x0 < g.nx) aa_odd_cell<DT, true, ACC>(p, a, x0, y, z, fxw, fzw, hit);
-        if (x0 + 1 < g.nx) aa_odd_cell<DT, true, ACC>(p, a, x0 + 1, y, z, fxw, fzw, hit);
-        if (((ka | kb) & TILE_FORCE) && p.force != nullptr) warp_force_add<float>(p, z, lane, fxw, fzw, hit);
-      } else {                                                        // odd: inlet, outlet, top
-        if (x0 < g.nx) aa_odd_cell<DT, false, ACC>(p, a, x0, y, z, fxw, fzw, hit);
-        if (x0 + 1 < g.nx) aa_odd_cell<DT, false, ACC>(p, a, x0 + 1, y, z, fxw, fzw, hit);
+        aa_pair_collide_scatter<DT, ACC>(p, v, x0, c, -row, row, lev, [&](int k) { return acc_box[k * 4 * 32]; });
       }
     }
   }
