@@ -17,7 +17,13 @@ from . import _native as N
 from .lattice import Q
 
 
+# the current stream's handle without a Stream object around it (0.3 instead of 3 us per launch)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream(stream=None):
+    if stream is None and _raw_stream is not None:
+        return ctypes.c_void_p(_raw_stream(torch.cuda.current_device()))
     s = stream if stream is not None else torch.cuda.current_stream()
     return ctypes.c_void_p(s.cuda_stream)
 

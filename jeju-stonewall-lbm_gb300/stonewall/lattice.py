@@ -37,10 +37,18 @@ MIRZ = np.array([int(np.flatnonzero((C == v * np.array([1, 1, -1])).all(1))[0]) 
 FLUID, WALL, GROUND = 0, 1, 2
 
 
+_TABLES = tuple((name, a, a.tobytes()) for name, a in
+                (("cx", np.ascontiguousarray(C[:, 0])), ("cy", np.ascontiguousarray(C[:, 1])),
+                 ("cz", np.ascontiguousarray(C[:, 2])), ("w", W), ("opp", OPP), ("mirz", MIRZ)))
+
+
 def check_tables(cx, cy, cz, w, opp, mirz):
-    """Raise ValueError unless the given arrays are this D3Q19 set (the kernels have it compiled in)."""
-    got = [np.asarray(a).ravel() for a in (cx, cy, cz, w, opp, mirz)]
-    want = [C[:, 0], C[:, 1], C[:, 2], W, OPP, MIRZ]
-    for name, g, e in zip(("cx", "cy", "cz", "w", "opp", "mirz"), got, want):
+    """Raise ValueError unless the given arrays are this D3Q19 set (the kernels have it compiled in).
+    The tables' own types are compared byte by byte, which a launch can afford; others by value."""
+    for (name, e, raw), g in zip(_TABLES, (cx, cy, cz, w, opp, mirz)):
+        g = np.asarray(g)
+        if g.dtype == e.dtype and g.shape == e.shape and g.tobytes() == raw:
+            continue
+        g = g.ravel()
         if g.shape != e.shape or not np.array_equal(g.astype(e.dtype), e):
             raise ValueError(f"lattice table {name} differs from the D3Q19 set compiled into the kernels")
