@@ -27,7 +27,7 @@ struct BatchCtx {
   const float *uin;
   double nu0, cs, nu_sponge, sponge_scale;
   float nu0f, c18f, sponge_scalef, nu_spongef;   // as StepParams (set_float_params)
-  double c18, tau0, tau0sq;                      // as StepParams (set_double_params)
+  double c18, tau0, tau0sq, sponge3;             // as StepParams (set_double_params)
   int x_sponge;
   long long *force;
   unsigned int *status;     // the lattice's status word, or nullptr

@@ -25,7 +25,7 @@
 // caller collides them in double.
 //
 // Error of one collision against 128-bit floats on the same inputs (25 kinds of
-// 20 000 cells, |u_a| up to 0.25, |Pi_neq| up to 3e-2): 4.6e-17 to 5.3e-17 of the
+// 20 000 cells, |u_a| up to 0.25, |Pi_neq| up to 3e-2): 4.6e-17 to 5.5e-17 of the
 // populations' norm, the rounding of the results included, against 1.4e-16 to
 // 1.6e-16 in double.
 //
@@ -63,7 +63,6 @@ __device__ __forceinline__ double dfma(double a, double b, double c) { return __
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double of_int(i64 v) { return __ll2double_rn(v); }
-__device__ __forceinline__ i64 to_int(double v) { return __double2ll_rn(v); }
 __device__ __forceinline__ double rcp_seed(double v) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(v));
@@ -83,7 +82,6 @@ inline double dfma(double a, double b, double c) { return std::fma(a, b, c); }
 inline double dmul(double a, double b) { return a * b; }
 inline double dadd(double a, double b) { return a + b; }
 inline double of_int(i64 v) { return (double)v; }
-inline i64 to_int(double v) { return v >= 9223372036854775807.0 ? 9223372036854775807ll : (i64)std::nearbyint(v); }
 // the device's seeds are within 2^-22 of the value; here that error is planted
 inline double rcp_seed(double v) { return (1.0 / v) * (1.0 + 2e-7); }
 inline double rsqrt_seed(double v) { return (1.0 / std::sqrt(v)) * (1.0 - 2e-7); }
@@ -110,14 +108,21 @@ __host__ __device__ __forceinline__ i64 to_units(double v, uint32_t emax, bool &
   return (i64)join(shl_hi(lo, m, t), lo << (t & 31u));
 }
 
-// v units (2^52 <= v < 2^62) as a double, rounded to nearest (ties up)
+// v units (2^40 <= v < 2^63) as a double, rounded to nearest (ties up)
 __host__ __device__ __forceinline__ double of_units(u64 v) {
   const uint32_t hi = hi32(v), lo = lo32(v);
-  const uint32_t s = (uint32_t)clz(hi);             // hi has a bit: s <= 11
+  const uint32_t s = (uint32_t)clz(hi);             // hi has a bit: s < 32
   const uint32_t nh = shl_hi(lo, hi, s), nl = lo << (s & 31u);
   // 53 bits with the leading one, which adds 1 to the exponent below; a carry out of them does so too
   const u64 r = (join(nh, nl) >> 11) + ((nl >> 10) & 1u);
   return of_bits(join(hi32(r) + ((1023u - s) << 20), lo32(r)));   // v = 2^(63 - s) 1.f units: exponent 1 - s
+}
+
+// A double in [1/4, 4) as a whole number of units, exact (2^-62 divides its last place).
+__host__ __device__ __forceinline__ i64 to_units_large(double v) {
+  const u64 b = bits_of(v);
+  const uint32_t t = (hi32(b) >> 20) - kExpMin, m = (hi32(b) & 0xfffffu) | 0x100000u;
+  return (i64)join(shl_hi(lo32(b), m, t), lo32(b) << (t & 31u));
 }
 
 // a b / 2^64, within 3 below
@@ -146,9 +151,8 @@ __host__ __device__ __forceinline__ double square_root(double v) {
 // new populations and mom rho and u (those are formed where they are used); false: the cell is out of range and
 // nothing of it is valid.
 struct Moments {
-  double r, y;                                      // rho 2^62 and its reciprocal
+  double rho;
   i64 u[3];                                         // u in units of 2^-61
-  __host__ __device__ __forceinline__ double rho() const { return scaled(r, -62); }
   __host__ __device__ __forceinline__ double vel(int k) const { return dmul(of_int(u[k]), 1.0 / 2305843009213693952.0); }
 };
 __host__ __device__ __forceinline__ bool collide(const double (&f)[19], double tau0, double tau0sq, double c18,
@@ -171,9 +175,9 @@ __host__ __device__ __forceinline__ bool collide(const double (&f)[19], double t
   const i64 mx = d[0] + (d[3] + d[4]) + (d[5] + d[6]);
   const i64 my = d[1] + (d[3] - d[4]) + (d[7] + d[8]);
   const i64 mz = d[2] + (d[5] - d[6]) + (d[7] - d[8]);
-  mom.r = of_int(rho);
-  mom.y = reciprocal(mom.r);
-  const i64 inv = to_int(scaled(mom.y, 124));       // 2^62 / rho in units of 2^-62: at most 2
+  mom.rho = of_units((u64)rho);
+  const double y = reciprocal(mom.rho);
+  const i64 inv = to_units_large(y);                // 1 / rho in (1/2, 2]
   // |m| < 3/4, |u| < 3/2: u and m u in units of 2^-61
   const i64 ux = mom.u[0] = mulhi(mx << 1, inv), uy = mom.u[1] = mulhi(my << 1, inv), uz = mom.u[2] = mulhi(mz << 1, inv);
   const i64 mx2 = mx << 1, my2 = my << 1, mz2 = mz << 1, ux2 = ux << 1, uy2 = uy << 1, uz2 = uz << 1;
@@ -195,11 +199,14 @@ __host__ __device__ __forceinline__ bool collide(const double (&f)[19], double t
     return (i64)(int)vh * (int)vh + (((i64)(int)vh * (int)(vl >> 1)) >> 30);
   };
   const i64 q = (square(nxx) + square(nyy) + square(nzz)) + ((square(nxy) + square(nxz) + square(nyz)) << 1);
-  const double qn = square_root(of_int(q | 1));     // |Pi_neq| 2^(30 + lead); never zero
-  const double c = scaled(dmul(c18, mom.y), 62 - 30 - lead);
-  const double root = square_root(dfma(c, qn, tau0sq));
-  // keep = 1 - 1 / tau, tau = (tau0 + root) / 2 > 1/2
-  const i64 keep = (1ll << 62) - to_int(scaled(reciprocal(dadd(tau0, root)), 63));
+  // below 2^40 only where every entry is below 2^-30: |Pi_neq| then counts as 2^-39, far below tau0's last place
+  const uint32_t qh = hi32((u64)q) < 256u ? 256u : hi32((u64)q);
+  const double qn = scaled(square_root(of_units(join(qh, lo32((u64)q)))), 1 - lead);
+  const double root = square_root(dfma(dmul(c18, y), qn, tau0sq));
+  // keep = 1 - 1 / tau, tau = (tau0 + root) / 2 > 1/2; tau of 4 and above is left to double
+  const double rt = scaled(reciprocal(dadd(tau0, root)), 1);
+  if (hi32(bits_of(rt)) < (1021u << 20)) return false;
+  const i64 keep = (i64)((1ull << 62) - (u64)to_units_large(rt));
   const i64 Bxx = bxx + mulhi(nxx << 1, keep), Byy = byy + mulhi(nyy << 1, keep), Bzz = bzz + mulhi(nzz << 1, keep);
   const i64 Bxy = bxy + mulhi(nxy << 1, keep), Bxz = bxz + mulhi(nxz << 1, keep), Byz = byz + mulhi(nyz << 1, keep);
   const i64 t = Bxx + Byy + Bzz;                    // B in units of 2^-61

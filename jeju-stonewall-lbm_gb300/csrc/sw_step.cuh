@@ -45,7 +45,7 @@ struct StepParams {
   // the host instead of converted from double in every thread
   float nu0f, c18f, sponge_scalef, nu_spongef;
   // the same for the float64 collision: 18 sqrt(2) Cs^2, 3 nu0 + 1/2 and its square (set_double_params)
-  double c18, tau0, tau0sq;
+  double c18, tau0, tau0sq, sponge3;   // (sponge3: 3 nu_sponge sponge_scale^2)
   int x_sponge;
   long long *force;  // force row of this step: [nz][2], or nullptr
   double *acc;       // float64 running sums [4][plane] (accumulation steps only)
@@ -98,6 +98,7 @@ template <typename P> __host__ __device__ inline void set_double_params(P &p) {
   p.c18 = 18.0 * sqrt(2.0) * p.cs * p.cs;
   p.tau0 = fma(3.0, p.nu0, 0.5);
   p.tau0sq = p.tau0 * p.tau0;
+  p.sponge3 = 3.0 * p.nu_sponge * p.sponge_scale * p.sponge_scale;
 }
 
 // Physics parameters in the collision's arithmetic type R.
@@ -244,9 +245,9 @@ __device__ __forceinline__ bool collide_cell(const Ctx &p, const R (&f)[Q], int 
   } else {
     static_assert(!SHIFT && sizeof(R) == 8, "fixed point takes float64 storage, which holds f itself");
     double tau0 = p.tau0, tau0sq = p.tau0sq;
-    if (x > p.x_sponge) {
-      const double sp = (double)(x - p.x_sponge) * ph.sponge_scale;
-      tau0 = fma(3.0, fma(ph.nu_sponge * sp, sp, ph.nu0), 0.5);
+    if (x > p.x_sponge) {                                       // nu = nu0 + nu_sponge ((x - x_sponge) scale)^2
+      const double dx = (double)(x - p.x_sponge);
+      tau0 = fma(p.sponge3, dx * dx, p.tau0);
       tau0sq = tau0 * tau0;
     }
     double out[Q];
@@ -254,7 +255,7 @@ __device__ __forceinline__ bool collide_cell(const Ctx &p, const R (&f)[Q], int 
     if (!fx::collide(f, tau0, tau0sq, ph.c18, out, m)) return false;
     static_for<0, Q>([&](auto I) { put(I, out[decltype(I)::value]); });
     if constexpr (WANT) {
-      rho = m.rho();
+      rho = m.rho;
       ux = m.vel(0);
       uy = m.vel(1);
       uz = m.vel(2);
@@ -273,10 +274,12 @@ template <int WY_, int MINB_> struct StepCfg {
   static constexpr int THREADS = 32 * WY_;
 };
 #define SW_STEP_CONFIGS(X) X(0, 8, 4) X(1, 8, 5) X(2, 4, 8) X(3, 4, 12)
-// The float64 step holds its 19 populations in register pairs: the same block
-// shapes with the registers that takes (128, 80, 96 and 80 per thread).
+// The float64 step holds its 19 populations in register pairs, and its long chains
+// of double operations want many warps in flight: the same block shapes with 64,
+// 48, 56 and 64 registers per thread (480x96x96: 0.266, 0.267, 0.261 and 0.260 ms
+// plain, 0.335, 0.382, 0.328 and 0.328 accumulating; with 96 registers 0.29).
 template <int DT, int WY, int MINB>
-using StepCfgOf = StepCfg<WY, DT != SW_F64 ? MINB : WY == 8 ? (MINB == 4 ? 2 : 3) : (MINB == 8 ? 5 : 6)>;
+using StepCfgOf = StepCfg<WY, DT != SW_F64 ? MINB : WY == 8 ? (MINB == 4 ? 4 : 5) : (MINB == 8 ? 9 : 8)>;
 // two cells per thread (16-bit storage only), see k_step_pair
 #define SW_PAIR_CONFIGS(X) X(4, 4, 8) X(5, 4, 10) X(6, 8, 4) X(7, 8, 5)
 // two cells per thread with TMA-staged sources (16-bit storage only), see sw_tma.cuh:

@@ -18,7 +18,7 @@ extern "C" void fx_cells(const double *f, int n, const double *tau0, const doubl
     ok[k] = sw::fx::collide(in, tau0[k], tau0[k] * tau0[k], c18[k], res, m);
     if (!ok[k]) continue;
     for (int i = 0; i < 19; ++i) out[19 * k + i] = res[i];
-    mom[4 * k] = m.rho();
+    mom[4 * k] = m.rho;
     for (int a = 0; a < 3; ++a) mom[4 * k + 1 + a] = m.vel(a);
   }
 }
