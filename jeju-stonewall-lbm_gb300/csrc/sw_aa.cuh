@@ -75,7 +75,7 @@ __device__ __noinline__ void aa_odd_cell_double(const StepParams &p, const AAPar
 template <int DT, bool CHECK, bool ACC>
 __device__ __noinline__ void aa_even_cell_double(const StepParams &p, int x, int y, int z);
 
-template <int DT, bool CHECK, bool ACC, bool FIXED = DT == SW_F64>
+template <int DT, bool CHECK, bool ACC, bool KEEP = false, bool FIXED = DT == SW_F64>
 __device__ __forceinline__ void aa_odd_cell(const StepParams &p, const AAParams &a, int x, int y, int z,
                                             typename Store<DT>::R &fxw, typename Store<DT>::R &fzw, int &hit) {
   using S = Store<DT>;
@@ -146,22 +146,23 @@ __device__ __forceinline__ void aa_odd_cell(const StepParams &p, const AAParams 
   // A segment without the checked path has only fluid neighbours around its
   // pulling cells; an inlet cell does not pull, so its targets are checked.
   const bool chk_t = CHECK || x == 0;
+  const Hold<KEEP> hold;
   auto scatter = [&](auto I, R v) {
     constexpr int k = decltype(I)::value;
     constexpr int ex = CX(k), ey = CY(k), ez = CZ(k);
     T *pl = p.template out<T>(k);
     const int oy = ey == 1 ? off_yp : ey == -1 ? off_ym : 0;   // row of y + c_y
     if (CHECK && (bounced >> OPP(k)) & 1u)                      // (d)
-      S::template st<k>(p.template out<T>(OPP(k)) + c, v);
+      S::template st<k>(p.template out<T>(OPP(k)) + c, v, hold);
     const int tx = x + ex, tz = z + ez;
     if (tx >= 0 && tx < g.nx && tz >= 0 && tz < g.nz) {          // (a)
       const int t = chk(p, c + ex + oy + ez * lev);
-      if (!chk_t || p.flag[t] == 0) S::template st<k>(pl + t, v);
+      if (!chk_t || p.flag[t] == 0) S::template st<k>(pl + t, v, hold);
     }
     if constexpr (ex == -1) {
       if (outlet && tz >= 0 && tz < g.nz) {                       // (b)
         const int t = chk(p, c + oy + ez * lev);
-        if (!chk_t || p.flag[t] == 0) S::template st<k>(pl + t, v);
+        if (!chk_t || p.flag[t] == 0) S::template st<k>(pl + t, v, hold);
       }
     }
     if constexpr (ez == 1) {
@@ -169,11 +170,11 @@ __device__ __forceinline__ void aa_odd_cell(const StepParams &p, const AAParams 
         T *pm = p.template out<T>(MIRZ(k));
         if (tx >= 0 && tx < g.nx) {
           const int t = chk(p, c + ex + oy);
-          if (!chk_t || p.flag[t] == 0) S::template st<MIRZ(k)>(pm + t, v);
+          if (!chk_t || p.flag[t] == 0) S::template st<MIRZ(k)>(pm + t, v, hold);
         }
         if (ex == -1 && outlet) {
           const int t = chk(p, c + oy);
-          if (!chk_t || p.flag[t] == 0) S::template st<MIRZ(k)>(pm + t, v);
+          if (!chk_t || p.flag[t] == 0) S::template st<MIRZ(k)>(pm + t, v, hold);
         }
       }
     }
@@ -208,7 +209,7 @@ __device__ __forceinline__ void aa_odd_cell(const StepParams &p, const AAParams 
   }
 }
 
-template <int DT, bool CHECK, bool ACC, bool FIXED = DT == SW_F64>
+template <int DT, bool CHECK, bool ACC, bool KEEP = false, bool FIXED = DT == SW_F64>
 __device__ __forceinline__ void aa_even_cell(const StepParams &p, int x, int y, int z, typename Store<DT>::R &fxw,
                                              typename Store<DT>::R &fzw, int &hit) {
   using S = Store<DT>;
@@ -219,9 +220,10 @@ __device__ __forceinline__ void aa_even_cell(const StepParams &p, int x, int y, 
   if (CHECK && p.flag[c] != 0) return;
   R rho, ux, uy, uz;
   // own cell: incoming values in natural slots (fin_pop), results to opposite slots (fout_pop is permuted)
+  const Hold<KEEP> hold;
   auto put = [&](auto I, R v) {
     constexpr int k = decltype(I)::value;
-    S::template st<k>(p.template out<T>(k) + c, v);
+    S::template st<k>(p.template out<T>(k) + c, v, hold);
   };
   if (x == 0) {
     const R u0 = (R)__ldg(p.uin + z);
@@ -284,16 +286,16 @@ template <int DT, bool CHECK, bool ACC>
 __device__ __noinline__ void aa_odd_cell_double(const StepParams &p, const AAParams &a, int x, int y, int z) {
   typename Store<DT>::R fxw(0), fzw(0);
   int hit = 0;
-  aa_odd_cell<DT, CHECK, ACC, false>(p, a, x, y, z, fxw, fzw, hit);
+  aa_odd_cell<DT, CHECK, ACC, false, false>(p, a, x, y, z, fxw, fzw, hit);
 }
 template <int DT, bool CHECK, bool ACC>
 __device__ __noinline__ void aa_even_cell_double(const StepParams &p, int x, int y, int z) {
   typename Store<DT>::R fxw(0), fzw(0);
   int hit = 0;
-  aa_even_cell<DT, CHECK, ACC, false>(p, x, y, z, fxw, fzw, hit);
+  aa_even_cell<DT, CHECK, ACC, false, false>(p, x, y, z, fxw, fzw, hit);
 }
 
-template <int DT, bool ODD, bool ACC, typename Cfg>
+template <int DT, bool ODD, bool ACC, bool KEEP, typename Cfg>
 __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) k_step_aa(const __grid_constant__ StepParams p, AAParams a) {
   using R = typename Store<DT>::R;
   const Geom &g = p.g;
@@ -308,14 +310,14 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB) k_step_aa(const __gri
   int hit = 0;
   if (!(kind & TILE_CHECK)) {
     if (x < g.nx) {
-      if (ODD) aa_odd_cell<DT, false, ACC>(p, a, x, y, z, fxw, fzw, hit);
-      else aa_even_cell<DT, false, ACC>(p, x, y, z, fxw, fzw, hit);
+      if (ODD) aa_odd_cell<DT, false, ACC, KEEP>(p, a, x, y, z, fxw, fzw, hit);
+      else aa_even_cell<DT, false, ACC, KEEP>(p, x, y, z, fxw, fzw, hit);
     }
     return;
   }
   if (x < g.nx) {
-    if (ODD) aa_odd_cell<DT, true, ACC>(p, a, x, y, z, fxw, fzw, hit);
-    else aa_even_cell<DT, true, ACC>(p, x, y, z, fxw, fzw, hit);
+    if (ODD) aa_odd_cell<DT, true, ACC, KEEP>(p, a, x, y, z, fxw, fzw, hit);
+    else aa_even_cell<DT, true, ACC, KEEP>(p, x, y, z, fxw, fzw, hit);
   }
   if ((kind & TILE_FORCE) && p.force != nullptr) warp_force_add<R>(p, z, lane, fxw, fzw, hit);
 }
@@ -501,9 +503,9 @@ __device__ __forceinline__ void tma_issue_own(const CUtensorMap *map, const CUte
   mbar_expect_tx(bar, Q * kTmaBoxBytes + (ACC ? kTmaAccBytes : 0));
   static_for<0, Q>([&](auto I) {
     constexpr int i = decltype(I)::value;
-    tma_load_4d(st + i * kTmaBoxBytes, map, x0 - 8, y0, z, OPP(i), bar);
+    tma_load_4d(st + i * kTmaBoxBytes, map, x0 - 8, y0, z, OPP(i), bar, Hold<false>{});
   });
-  if constexpr (ACC) tma_load_4d(st + kTmaStageBytes, map_acc, x0, y0, z, 0, bar);
+  if constexpr (ACC) tma_load_4d(st + kTmaStageBytes, map_acc, x0, y0, z, 0, bar, Hold<false>{});
 }
 
 // The populations with c_x = -1 that the outlet cell of (y, z) pulls: column nx - 1 before the step (the ghost).
@@ -735,7 +737,7 @@ __device__ __forceinline__ void aa_odd_pair_checked(const StepParams &p, const u
   if (force && p.force != nullptr) warp_force_add<float>(p, z, lane, fxw, fzw, hit);
 }
 
-template <int DT, bool ODD, bool ACC>
+template <int DT, bool ODD, bool ACC, bool KEEP>
 __global__ void __launch_bounds__(128, 9)
     k_step_aa_tma(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap map1,
                   const __grid_constant__ CUtensorMap map_acc, const __grid_constant__ StepParams p, AAParams a) {
@@ -819,7 +821,7 @@ __global__ void __launch_bounds__(128, 9)
           const uint32_t keep = pair_solid_cells(v, sm);
           if (keep != 0u) {
             const double2 *acc_box = reinterpret_cast<const double2 *>(smem + kTmaStageBytes) + w * 32 + lane;
-            pair_collide_store<DT, ACC, true>(p, v, x0, c, z, x0 == 0, has_b,
+            pair_collide_store<DT, ACC, true, KEEP>(p, v, x0, c, z, x0 == 0, has_b,
                                               [&](int k) { return acc_box[k * 4 * 32]; }, keep);
           }
         }
@@ -834,7 +836,7 @@ __global__ void __launch_bounds__(128, 9)
             v[i].v = PK::both(reinterpret_cast<const uint32_t *>(smem + i * kTmaBoxBytes + w * kTmaRowBytes)[lane_word]);
           });
           const double2 *acc_box = reinterpret_cast<const double2 *>(smem + kTmaStageBytes) + w * 32 + lane;
-          pair_collide_store<DT, ACC>(p, v, x0, c, z, x0 == 0, has_b, [&](int k) { return acc_box[k * 4 * 32]; });
+          pair_collide_store<DT, ACC, false, KEEP>(p, v, x0, c, z, x0 == 0, has_b, [&](int k) { return acc_box[k * 4 * 32]; });
         }
       }
     } else {
@@ -872,6 +874,19 @@ __global__ void __launch_bounds__(128, 9)
   }
 }
 
+// Whether an in-place step holds lines in L2.  The 16-bit even step (whose stores
+// are whole words): lattices well above the L2 (us per step, streaming / held, odd
+// and even together: 480x96x96, 168 MB, 77.9 / 78.7; 520x104x104 94.2 / 93.2;
+// 640x128x128 157 / 152; 800x160x160 299 / 286).  float32: where the one lattice
+// fits the L2 (320x64x64 35.4 / 30.6) and from about 300 MB (800x160x160 498 /
+// 496); between them only the accumulating steps (420x84x84 plain 80.9 / 82.1,
+// accumulating 88.1 / 87.9).
+template <int DT> inline bool hold_aa(const StepParams &p) {
+  const long long bytes = p.g.plane * Q * (long long)sizeof(typename Store<DT>::T);
+  if (is16(DT)) return bytes > 180000000ll;
+  return DT == SW_F32 && (p.acc != nullptr || bytes < 126000000ll || bytes > 300000000ll);
+}
+
 // The TMA-staged AA step on the lattice p.fin (== p.fout); cudaErrorNotSupported
 // when the tensor maps cannot be made (the caller then runs k_step_aa_pair).
 template <int DT, bool ODD, bool ACC>
@@ -887,7 +902,8 @@ cudaError_t launch_aa_tma(const StepParams &p, const AAParams &a, cudaStream_t s
   constexpr int smem = tma_stage_bytes<ACC>() + 128;
   static_assert(smem <= 48 * 1024, "one stage fits the default shared memory of a block");
   const dim3 grid((unsigned)((p.g.nseg_x + 1) / 2), (unsigned)((p.g.ny + 3) / 4), (unsigned)p.g.nz);
-  k_step_aa_tma<DT, ODD, ACC><<<grid, dim3(32, 4), smem, s>>>(map, map1, map_acc, p, a);
+  if (!ODD && hold_aa<DT>(p)) k_step_aa_tma<DT, ODD, ACC, !ODD><<<grid, dim3(32, 4), smem, s>>>(map, map1, map_acc, p, a);
+  else k_step_aa_tma<DT, ODD, ACC, false><<<grid, dim3(32, 4), smem, s>>>(map, map1, map_acc, p, a);
   return cudaGetLastError();
 }
 
@@ -938,12 +954,17 @@ cudaError_t launch_aa(const StepParams &p_in, const AAParams &a, bool odd, cudaS
     using Cfg = decltype(cfg);
     const dim3 grid((unsigned)p.g.nseg_x, (unsigned)((p.g.ny + Cfg::WY - 1) / Cfg::WY), (unsigned)p.g.nz);
     const dim3 block(32, Cfg::WY);
-    if (odd) {
-      if (p.acc) k_step_aa<DT, true, true, Cfg><<<grid, block, 0, s>>>(p, a);
-      else k_step_aa<DT, true, false, Cfg><<<grid, block, 0, s>>>(p, a);
+    constexpr bool K = DT == SW_F32;                  // (float64 has no held form)
+    if (K && hold_aa<DT>(p)) {
+      if (odd && p.acc) k_step_aa<DT, true, true, K, Cfg><<<grid, block, 0, s>>>(p, a);
+      else if (odd) k_step_aa<DT, true, false, K, Cfg><<<grid, block, 0, s>>>(p, a);
+      else if (p.acc) k_step_aa<DT, false, true, K, Cfg><<<grid, block, 0, s>>>(p, a);
+      else k_step_aa<DT, false, false, K, Cfg><<<grid, block, 0, s>>>(p, a);
     } else {
-      if (p.acc) k_step_aa<DT, false, true, Cfg><<<grid, block, 0, s>>>(p, a);
-      else k_step_aa<DT, false, false, Cfg><<<grid, block, 0, s>>>(p, a);
+      if (odd && p.acc) k_step_aa<DT, true, true, false, Cfg><<<grid, block, 0, s>>>(p, a);
+      else if (odd) k_step_aa<DT, true, false, false, Cfg><<<grid, block, 0, s>>>(p, a);
+      else if (p.acc) k_step_aa<DT, false, true, false, Cfg><<<grid, block, 0, s>>>(p, a);
+      else k_step_aa<DT, false, false, false, Cfg><<<grid, block, 0, s>>>(p, a);
     }
     return cudaGetLastError();
   };

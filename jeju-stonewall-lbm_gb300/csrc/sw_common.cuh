@@ -62,6 +62,40 @@ enum : uint8_t {
 // the per-level totals do not depend on the order in which warps finish.
 constexpr double FORCE_SCALE = 1099511627776.0;  // 2^40
 
+// ---------------------------------------------------------------- L2 eviction
+// How a step stores the new populations: streaming (st.cs), or with L2 eviction
+// priority evict_last (Hold<true>), which keeps written lines until runs of them
+// go to DRAM together, at the price of a policy operand on every store.
+// float32 two-lattice steps hold at every size (us per step, streaming / held):
+// 240x48x48 11.6 / 11.1, 320x64x64 33.2 / 31.9, 480x96x96 104.9 / 101.6,
+// 800x160x160 461 / 453.  float64 does not: its step is short of registers
+// (480x96x96 257 / 263).  The 16-bit and in-place steps choose by size
+// (hold_pair16, hold_aa).
+template <bool KEEP> struct Hold {};
+template <> struct Hold<true> {
+  uint64_t policy;
+  __device__ __forceinline__ Hold() {
+    asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(policy));
+  }
+};
+template <typename T> __device__ __forceinline__ void st_new(T *q, T v, const Hold<false> &) { __stcs(q, v); }
+__device__ __forceinline__ void st_new(float *q, float v, const Hold<true> &h) {
+  asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(q), "f"(v), "l"(h.policy) : "memory");
+}
+__device__ __forceinline__ void st_new(double *q, double v, const Hold<true> &h) {
+  asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;" ::"l"(q), "d"(v), "l"(h.policy) : "memory");
+}
+__device__ __forceinline__ void st_new(unsigned int *q, unsigned int v, const Hold<true> &h) {
+  asm volatile("st.global.L2::cache_hint.b32 [%0], %1, %2;" ::"l"(q), "r"(v), "l"(h.policy) : "memory");
+}
+template <typename H16> __device__ __forceinline__ void st_new16(H16 *q, H16 v, const Hold<true> &h) {
+  asm volatile("st.global.L2::cache_hint.b16 [%0], %1, %2;" ::"l"(q), "h"(*reinterpret_cast<const uint16_t *>(&v)),
+               "l"(h.policy)
+               : "memory");
+}
+__device__ __forceinline__ void st_new(__half *q, __half v, const Hold<true> &h) { st_new16(q, v, h); }
+__device__ __forceinline__ void st_new(__nv_bfloat16 *q, __nv_bfloat16 v, const Hold<true> &h) { st_new16(q, v, h); }
+
 // ---------------------------------------------------------------- storage policies
 // R = arithmetic type of the collision, T = stored type.  The shifted 16-bit
 // formats store g_i = f_i - w_i (the deviation from the rest state) to keep the
@@ -75,7 +109,7 @@ template <> struct Store<SW_F32> {
   using R = float;
   static constexpr bool kShift = false;
   template <int I> static __device__ __forceinline__ R ld(const T *p) { return __ldg(p); }
-  template <int I> static __device__ __forceinline__ void st(T *p, R v) { __stcs(p, v); }
+  template <int I, typename H> static __device__ __forceinline__ void st(T *p, R v, const H &h) { st_new(p, v, h); }
   template <int I> static __device__ __forceinline__ T enc(R v) { return v; }
   template <int I> static __device__ __forceinline__ R dec(T v) { return v; }
 };
@@ -84,7 +118,7 @@ template <> struct Store<SW_F64> {
   using R = double;
   static constexpr bool kShift = false;
   template <int I> static __device__ __forceinline__ R ld(const T *p) { return __ldg(p); }
-  template <int I> static __device__ __forceinline__ void st(T *p, R v) { __stcs(p, v); }
+  template <int I, typename H> static __device__ __forceinline__ void st(T *p, R v, const H &h) { st_new(p, v, h); }
   template <int I> static __device__ __forceinline__ T enc(R v) { return v; }
   template <int I> static __device__ __forceinline__ R dec(T v) { return v; }
 };
@@ -95,7 +129,9 @@ template <> struct Store<SW_F16_SHIFT> {
   template <int I> static __device__ __forceinline__ R dec(T v) { return W<float>(I) + __half2float(v); }
   template <int I> static __device__ __forceinline__ T enc(R v) { return __float2half_rn(v - W<float>(I)); }
   template <int I> static __device__ __forceinline__ R ld(const T *p) { return __half2float(__ldg(p)); }
-  template <int I> static __device__ __forceinline__ void st(T *p, R v) { __stcs(p, __float2half_rn(v)); }
+  template <int I, typename H> static __device__ __forceinline__ void st(T *p, R v, const H &h) {
+    st_new(p, __float2half_rn(v), h);
+  }
   static __device__ __forceinline__ T from_shifted(R g) { return __float2half_rn(g); }
   static __device__ __forceinline__ R to_shifted(T v) { return __half2float(v); }
 };
@@ -106,7 +142,9 @@ template <> struct Store<SW_BF16_SHIFT> {
   template <int I> static __device__ __forceinline__ R dec(T v) { return W<float>(I) + __bfloat162float(v); }
   template <int I> static __device__ __forceinline__ T enc(R v) { return __float2bfloat16_rn(v - W<float>(I)); }
   template <int I> static __device__ __forceinline__ R ld(const T *p) { return __bfloat162float(__ldg(p)); }
-  template <int I> static __device__ __forceinline__ void st(T *p, R v) { __stcs(p, __float2bfloat16_rn(v)); }
+  template <int I, typename H> static __device__ __forceinline__ void st(T *p, R v, const H &h) {
+    st_new(p, __float2bfloat16_rn(v), h);
+  }
   static __device__ __forceinline__ T from_shifted(R g) { return __float2bfloat16_rn(g); }
   static __device__ __forceinline__ R to_shifted(T v) { return __bfloat162float(v); }
 };

@@ -350,6 +350,7 @@ __device__ __forceinline__ void step_cell(const Ctx &p, int x, int y, int z, typ
   const int c = chk(p, (z * g.ny + y) * g.pitch + x);
   auto out = [&](int pop) { return p.template out<T>(pop); };
   if (CHECK && pull_val.self_solid(p, c)) return;              // lbm3d.py:65-66
+  const Hold<DT == SW_F32> hold;
   if (x == 0) {                                                 // inlet, lbm3d.py:67-71
     const R u0 = (R)__ldg(p.uin + z);
     const R usq = u0 * u0;
@@ -360,7 +361,7 @@ __device__ __forceinline__ void step_cell(const Ctx &p, int x, int y, int z, typ
       if constexpr (ex != 0) cu = (ex > 0 ? u0 : -u0);
       cu = R(3.0) * cu;
       const R v = W<R>(i) * R(1.0) * (R(1.0) + cu + R(0.5) * cu * cu - R(1.5) * usq);
-      S::template st<i>(out(i) + c, S::kShift ? v - W<R>(i) : v);
+      S::template st<i>(out(i) + c, S::kShift ? v - W<R>(i) : v, hold);
     });
     if (ACC) {
       atomicAdd(p.accp(0) + c, 1.0);
@@ -418,7 +419,7 @@ __device__ __forceinline__ void step_cell(const Ctx &p, int x, int y, int z, typ
   R rho, ux, uy, uz;
   const bool done = collide_cell<R, S::kShift, ACC, FIXED>(p, fl, x, rho, ux, uy, uz, [&](auto I, R v) {
     constexpr int i = decltype(I)::value;
-    S::template st<i>(out(i) + c, v);
+    S::template st<i>(out(i) + c, v, hold);
   });
   if constexpr (FIXED) {
     if (!done) {                                                // nothing written yet; the force is summed already
@@ -739,24 +740,26 @@ __device__ __forceinline__ uint32_t pair_solid_cells(f2 (&v)[Q], const uint32_t 
 // of the pair for sum k (a double2; .y unused without has_b), called where
 // they are added.  MASKED (the checked path): only the cells in `keep` (bit 0:
 // x0, bit 1: x0 + 1) are stored and summed; the inlet cell only when kept.
-template <int DT, bool ACC, bool MASKED = false, typename Ctx, typename AccOld>
+// KEEP: the stores hold their lines in L2.
+template <int DT, bool ACC, bool MASKED = false, bool KEEP = false, typename Ctx, typename AccOld>
 __device__ __forceinline__ void pair_collide_store(const Ctx &p, const f2 (&v)[Q], int x0, int c, int z, bool inlet,
                                                    bool has_b, AccOld &&acc_old, uint32_t keep = 3u) {
   using S = Store<DT>;
   using T = typename S::T;
   using PK = Pack16<DT>;
   const Phys<float> ph = phys<float>(p);
+  const Hold<KEEP> hold;
   f2 rho, ux, uy, uz;
   if (MASKED) inlet = inlet && (keep & 1u);
   collide2(v, x0, has_b, ph.nu0, ph.c18, p.x_sponge, ph.sponge_scale, ph.nu_sponge, rho, ux, uy, uz,
            p.status, [&](auto I, f2 o) {
              constexpr int i = decltype(I)::value;
              if (!MASKED || keep == 3u)
-               __stcs(reinterpret_cast<unsigned int *>(p.template out<T>(i) + c), PK::pack(o.v.x, o.v.y));
+               st_new(reinterpret_cast<unsigned int *>(p.template out<T>(i) + c), PK::pack(o.v.x, o.v.y), hold);
              else if (keep == 1u)
-               __stcs(p.template out<T>(i) + c, S::from_shifted(o.v.x));
+               st_new(p.template out<T>(i) + c, S::from_shifted(o.v.x), hold);
              else if (keep == 2u)
-               __stcs(p.template out<T>(i) + c + 1, S::from_shifted(o.v.y));
+               st_new(p.template out<T>(i) + c + 1, S::from_shifted(o.v.y), hold);
            });
   float u0 = 0.0f;
   if (inlet) {
@@ -769,7 +772,7 @@ __device__ __forceinline__ void pair_collide_store(const Ctx &p, const f2 (&v)[Q
       if constexpr (ex != 0) cu = (ex > 0 ? u0 : -u0);
       cu = 3.0f * cu;
       const float w = W<float>(i) * 1.0f * (1.0f + cu + 0.5f * cu * cu - 1.5f * usq);
-      __stcs(p.template out<T>(i) + c, S::from_shifted(w - W<float>(i)));
+      st_new(p.template out<T>(i) + c, S::from_shifted(w - W<float>(i)), hold);
     });
   }
   if (ACC) {

@@ -100,20 +100,29 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int pol
   return false;
 }
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, int c3,
-                                            uint32_t bar) {
+                                            uint32_t bar, const Hold<false> &) {
   asm volatile(
       "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
       "[%6];" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
       : "memory");
 }
-
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, int c3,
+                                            uint32_t bar, const Hold<true> &hold) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, "
+      "%3, %4, %5}], [%6], %7;" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar), "l"(hold.policy)
+      : "memory");
+}
 
 // Issue the copies of item (x0, y0, z) into stage `st`, arriving on `bar` (one
 // thread); with ACC also the item's float64 sums (map_acc) behind the boxes.
-template <bool ACC>
+// KEEP: the copies hold their lines in L2, as the stores do.
+template <bool ACC, bool KEEP = false>
 __device__ __forceinline__ void tma_issue(const CUtensorMap *map, const CUtensorMap *map1, const CUtensorMap *map_acc,
                                           const Geom &g, int x0, int y0, int z, uint32_t st, uint32_t bar) {
+  const Hold<KEEP> hold;
   const bool top = z == g.nz - 1;
   const bool wrap_lo = y0 == 0;                  // source row -1 of the first warp (c_y = +1)
   const bool wrap_hi = y0 + 4 >= g.ny;           // source row ny of the warp at y = ny - 1 (c_y = -1)
@@ -126,14 +135,14 @@ __device__ __forceinline__ void tma_issue(const CUtensorMap *map, const CUtensor
     constexpr int ey = CY(i), ez = CZ(i);
     const int pop = (ez == -1 && top) ? MIRZ(i) : i;
     const int zl = (ez == -1 && top) ? z : z - ez;
-    tma_load_4d(st + i * kTmaBoxBytes, map, x0 - 8, y0 - ey, zl, pop, bar);
+    tma_load_4d(st + i * kTmaBoxBytes, map, x0 - 8, y0 - ey, zl, pop, bar, hold);
     if constexpr (ey == 1) {
-      if (wrap_lo) tma_load_4d(st + Q * kTmaBoxBytes + wrap_slot(i) * kTmaWrapBytes, map1, x0 - 8, g.ny - 1, zl, pop, bar);
+      if (wrap_lo) tma_load_4d(st + Q * kTmaBoxBytes + wrap_slot(i) * kTmaWrapBytes, map1, x0 - 8, g.ny - 1, zl, pop, bar, hold);
     } else if constexpr (ey == -1) {
-      if (wrap_hi) tma_load_4d(st + Q * kTmaBoxBytes + wrap_slot(i) * kTmaWrapBytes, map1, x0 - 8, 0, zl, pop, bar);
+      if (wrap_hi) tma_load_4d(st + Q * kTmaBoxBytes + wrap_slot(i) * kTmaWrapBytes, map1, x0 - 8, 0, zl, pop, bar, hold);
     }
   });
-  if constexpr (ACC) tma_load_4d(st + kTmaStageBytes, map_acc, x0, y0, z, 0, bar);
+  if constexpr (ACC) tma_load_4d(st + kTmaStageBytes, map_acc, x0, y0, z, 0, bar, hold);
 }
 
 // The pair-kernel two-cell step with the sources read from the staged boxes (st: the stage).
@@ -142,7 +151,7 @@ __device__ __forceinline__ void tma_issue(const CUtensorMap *map, const CUtensor
 // so no lane needs the inlet, outlet or wrap selects (decided per warp and item).
 // CHECKED: as step_pair_fast's (link masks and bounce-back pairs from
 // pair_links_prefetch; the boxes read zeros below z = 0).
-template <int DT, bool ACC, bool INTERIOR, bool CHECKED = false>
+template <int DT, bool ACC, bool INTERIOR, bool KEEP, bool CHECKED = false>
 __device__ __forceinline__ void tma_pair_fast(const StepParams &p, const uint8_t *st, int x0, int y, int z, int w,
                                               int lane, const uint32_t (*sm)[2] = nullptr,
                                               const uint32_t (*wm)[2] = nullptr, const uint32_t (*bnc)[Q] = nullptr,
@@ -186,14 +195,15 @@ __device__ __forceinline__ void tma_pair_fast(const StepParams &p, const uint8_t
   if constexpr (CHECKED) {
     const uint32_t keep = pair_solid_cells(v, *sm);
     if (keep == 0u) return;
-    pair_collide_store<DT, ACC, true>(p, v, x0, c, z, inlet, has_b, [&](int k) { return acc_box[k * 4 * 32]; }, keep);
+    pair_collide_store<DT, ACC, true, KEEP>(p, v, x0, c, z, inlet, has_b, [&](int k) { return acc_box[k * 4 * 32]; },
+                                             keep);
   } else {
-    pair_collide_store<DT, ACC>(p, v, x0, c, z, inlet, has_b, [&](int k) { return acc_box[k * 4 * 32]; });
+    pair_collide_store<DT, ACC, false, KEEP>(p, v, x0, c, z, inlet, has_b, [&](int k) { return acc_box[k * 4 * 32]; });
   }
 }
 
 // Grid: (ceil(pitch / 64), ceil(ceil(ny / 4) / ITEMS), nz); block = 4 warps, warp w = row y0 + w.
-template <int DT, bool ACC, typename Cfg>
+template <int DT, bool ACC, typename Cfg, bool KEEP>
 __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
     k_step_tma(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap map1,
                const __grid_constant__ CUtensorMap map_acc, const __grid_constant__ StepParams p) {
@@ -219,7 +229,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     for (int j = 0; j < Cfg::NSTAGE && j < n_items; ++j)
-      tma_issue<ACC>(&map, &map1, &map_acc, g, x0s, (yb0 + j) * 4, z, base + j * kStage, smem_u32(&bars[j]));
+      tma_issue<ACC, KEEP>(&map, &map1, &map_acc, g, x0s, (yb0 + j) * 4, z, base + j * kStage, smem_u32(&bars[j]));
   }
   // The segment classes of this warp's rows in all its items, fetched once up
   // front (lane j: segment 2 bx of item j, lane ITEMS + j: segment 2 bx + 1),
@@ -251,13 +261,14 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
     if (ok && work) {
       if (!checked) {
         if (x0s > 0 && x0s + 2 * SEG < g.nx && y > 0 && y < g.ny - 1)     // uniform across the warp
-          tma_pair_fast<DT, ACC, true>(p, smem + s * kStage, x0, y, z, w, lane);
+          tma_pair_fast<DT, ACC, true, KEEP>(p, smem + s * kStage, x0, y, z, w, lane);
         else
-          tma_pair_fast<DT, ACC, false>(p, smem + s * kStage, x0, y, z, w, lane);
+          tma_pair_fast<DT, ACC, false, KEEP>(p, smem + s * kStage, x0, y, z, w, lane);
       } else {                                                        // next to stones / the ground
         float fxw = 0.0f, fzw = 0.0f;
         int hit = 0;
-        tma_pair_fast<DT, ACC, false, true>(p, smem + s * kStage, x0, y, z, w, lane, &sm, &wm, &bnc, &fxw, &fzw, &hit);
+        tma_pair_fast<DT, ACC, false, KEEP, true>(p, smem + s * kStage, x0, y, z, w, lane, &sm, &wm, &bnc, &fxw, &fzw,
+                                                  &hit);
         if (((ka | kb) & TILE_FORCE) && p.force != nullptr) warp_force_add<float>(p, z, lane, fxw, fzw, hit);
       }
     }
@@ -265,7 +276,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
       ok = __syncthreads_and(ok);                                     // barrier frees stage s
       if (!ok) break;
       if (leader && j + Cfg::NSTAGE < n_items)
-        tma_issue<ACC>(&map, &map1, &map_acc, g, x0s, (yb0 + j + Cfg::NSTAGE) * 4, z, st, smem_u32(&bars[s]));
+        tma_issue<ACC, KEEP>(&map, &map1, &map_acc, g, x0s, (yb0 + j + Cfg::NSTAGE) * 4, z, st, smem_u32(&bars[s]));
     }
   }
   if constexpr (!kRing) ok = __syncthreads_and(ok);                 // every item was issued at the start
@@ -320,8 +331,15 @@ inline bool encode_acc_map(CUtensorMap *m, const double *acc, const Geom &g) {
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int DT, bool ACC, typename Cfg>
-cudaError_t launch_tma(const StepParams &p, cudaStream_t s) {
+// Whether a 16-bit two-lattice step holds lines in L2: once the lattice pair
+// exceeds the L2 (us per step, streaming / held: 280x56x56, 67 MB a pair, 13.0 /
+// 13.5; 320x64x64, 100 MB, 17.8 / 18.0; 352x68x68, 124 MB, 26.1 / 25.8; 360x72x72,
+// 145 MB, 29.7 / 28.8; 440x88x88 48.0 / 46.2; 800x160x160 245 / 243, accumulating
+// 281 / 278).
+inline bool hold_pair16(const Geom &g) { return g.plane * (2ll * Q * 2) > 118000000ll; }
+
+template <int DT, bool ACC, typename Cfg, bool KEEP>
+cudaError_t launch_tma_as(const StepParams &p, cudaStream_t s) {
   CUtensorMap map, map1, map_acc;
   if (!encode_lattice_map(&map, p.fin, p.g, 4) || !encode_lattice_map(&map1, p.fin, p.g, 1))
     return cudaErrorNotSupported;
@@ -335,7 +353,7 @@ cudaError_t launch_tma(const StepParams &p, cudaStream_t s) {
   if constexpr (smem > 48 * 1024) {                                  // beyond the default: opt in, once
     static bool opted = false;
     if (!opted) {
-      const cudaError_t e = cudaFuncSetAttribute(k_step_tma<DT, ACC, Cfg>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      const cudaError_t e = cudaFuncSetAttribute(k_step_tma<DT, ACC, Cfg, KEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  smem);
       if (e != cudaSuccess) return e;
       opted = true;
@@ -343,8 +361,13 @@ cudaError_t launch_tma(const StepParams &p, cudaStream_t s) {
   }
   const int nyb = (p.g.ny + 3) / 4;
   const dim3 grid((unsigned)((p.g.nseg_x + 1) / 2), (unsigned)((nyb + Cfg::ITEMS - 1) / Cfg::ITEMS), (unsigned)p.g.nz);
-  k_step_tma<DT, ACC, Cfg><<<grid, dim3(32, 4), smem, s>>>(map, map1, map_acc, p);
+  k_step_tma<DT, ACC, Cfg, KEEP><<<grid, dim3(32, 4), smem, s>>>(map, map1, map_acc, p);
   return cudaGetLastError();
+}
+
+template <int DT, bool ACC, typename Cfg>
+cudaError_t launch_tma(const StepParams &p, cudaStream_t s) {
+  return hold_pair16(p.g) ? launch_tma_as<DT, ACC, Cfg, true>(p, s) : launch_tma_as<DT, ACC, Cfg, false>(p, s);
 }
 
 }  // namespace sw
