@@ -79,6 +79,12 @@ def acc_steps(t0, n, n_spin, every):
     return 0 if first >= hi else (hi - 1 - first) // every + 1
 
 
+# The persistent kernel's configuration unless one is given or tuned.  Blocks of eight rows take the
+# items in longer runs; they are the fastest for float32 in every mix measured (us per step,
+# configuration 1 / 3: six walls of H 12-24 324 / 347, two of H 40 1033 / 1091, twelve of H 8 77 / 83,
+# one of H 16 44 / 50).  float64 wants 3 (six walls 786 against 801-917), 16 bits 4 (259 against 265).
+_DEFAULT_CFG = {N.SW_F32: 1, N.SW_F64: 3, N.SW_F16_SHIFT: 4, N.SW_BF16_SHIFT: 4}
+
 GRAPH_MAX = 256          # SW_BATCH_MAX_ENTRIES: lattices per sw_batch_graph_run
 
 
@@ -89,7 +95,7 @@ class Batch:
         self.chunk = int(chunk)
         self.max_members = int(max_members)
         self.members = []
-        self.cfg = cfg if cfg is not None else (4 if self.dtype in (N.SW_F16_SHIFT, N.SW_BF16_SHIFT) else 3)
+        self.cfg = cfg if cfg is not None else _DEFAULT_CFG[self.dtype]
         esz = ctypes.sizeof(SwBatchEntry)
         self._table_dev = torch.zeros(self.max_members * esz, dtype=torch.uint8, device=self.device)
         self._hdr_dev = torch.zeros(ctypes.sizeof(SwBatchHeader), dtype=torch.uint8, device=self.device)
