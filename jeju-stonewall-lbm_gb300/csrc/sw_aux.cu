@@ -245,97 +245,128 @@ __global__ void __launch_bounds__(256) k_build_tiles(Geom g, const uint8_t *flag
 
 // ---------------------------------------------------------------- x <-> z transposes
 // Reference layout a[k][x][y][z] (z fastest) <-> device layout b[k][z][y][pitch].
-// One block moves a 32 x 32 tile of the (x, z) plane of one (k, y).
+// One block moves a 64 x 32 tile of the (x, z) plane of one (k, y), eight elements
+// per thread in flight on either side.  Bound by DRAM; with one element in flight
+// per row step (32 x 32 tiles) and the weight of k found per element, a float32
+// 480x96x96 lattice took 240 us each way, now 139.
+constexpr int kTileX = 64, kTileZ = 32, kTileThreads = 256;
 template <typename A, typename B, typename Conv>
-__global__ void k_ref_to_dev(Geom g, int nk, const A *a, B *b, Conv conv) {
-  __shared__ A t[32][33];
+__global__ void __launch_bounds__(kTileThreads) k_ref_to_dev(Geom g, const A *a, B *b, Conv make) {
+  __shared__ A t[kTileX][kTileZ + 1];
   const int ky = blockIdx.x;             // k * ny + y
   const int k = ky / g.ny, y = ky % g.ny;
-  const int x0 = blockIdx.y * 32, z0 = blockIdx.z * 32;
-  const size_t aplane = (size_t)g.nx * g.ny * g.nz;
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {   // r: x offset, threadIdx.x: z offset
-    const int x = x0 + r, z = z0 + threadIdx.x;
-    if (x < g.nx && z < g.nz) t[r][threadIdx.x] = a[k * aplane + ((size_t)x * g.ny + y) * g.nz + z];
+  const int x0 = blockIdx.y * kTileX, z0 = blockIdx.z * kTileZ;
+  const auto conv = make(k);
+  constexpr int kRows = kTileThreads / kTileZ, N = kTileX / kRows;
+  {
+    const int dz = threadIdx.x % kTileZ, dx = threadIdx.x / kTileZ, z = z0 + dz;
+    const A *src = a + (size_t)k * g.nx * g.ny * g.nz + ((size_t)(x0 + dx) * g.ny + y) * g.nz + z;
+    A v[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if (x0 + dx + j * kRows < g.nx && z < g.nz) v[j] = __ldg(src + (size_t)j * kRows * g.ny * g.nz);
+#pragma unroll
+    for (int j = 0; j < N; ++j) t[dx + j * kRows][dz] = v[j];
   }
   __syncthreads();
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {   // r: z offset, threadIdx.x: x offset
-    const int z = z0 + r, x = x0 + threadIdx.x;
-    if (x < g.pitch && z < g.nz) {
-      const size_t o = (size_t)k * g.plane + ((size_t)z * g.ny + y) * g.pitch + x;
-      if (x < g.nx) b[o] = conv(k, t[threadIdx.x][r]);
-      else b[o] = conv.pad(k);
-    }
-  }
-  (void)nk;
+  constexpr int kLevels = kTileThreads / kTileX, M = kTileZ / kLevels;
+  const int dx = threadIdx.x % kTileX, dz = threadIdx.x / kTileX, x = x0 + dx;
+  if (x >= g.pitch) return;
+  B *dst = b + (size_t)k * g.plane + ((size_t)(z0 + dz) * g.ny + y) * g.pitch + x;
+#pragma unroll
+  for (int j = 0; j < M; ++j)
+    if (z0 + dz + j * kLevels < g.nz)
+      dst[(size_t)j * kLevels * g.ny * g.pitch] = x < g.nx ? conv(t[dx][dz + j * kLevels]) : conv.pad();
 }
 
 template <typename B, typename A, typename Conv>
-__global__ void k_dev_to_ref(Geom g, int nk, const B *b, A *a, Conv conv) {
-  __shared__ A t[32][33];
+__global__ void __launch_bounds__(kTileThreads) k_dev_to_ref(Geom g, const B *b, A *a, Conv make) {
+  __shared__ A t[kTileX][kTileZ + 1];
   const int ky = blockIdx.x;
   const int k = ky / g.ny, y = ky % g.ny;
-  const int x0 = blockIdx.y * 32, z0 = blockIdx.z * 32;
-  const size_t aplane = (size_t)g.nx * g.ny * g.nz;
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {   // r: z offset, threadIdx.x: x offset
-    const int z = z0 + r, x = x0 + threadIdx.x;
-    if (x < g.nx && z < g.nz) t[r][threadIdx.x] = conv(k, b[(size_t)k * g.plane + ((size_t)z * g.ny + y) * g.pitch + x]);
+  const int x0 = blockIdx.y * kTileX, z0 = blockIdx.z * kTileZ;
+  const auto conv = make(k);
+  {
+    constexpr int kLevels = kTileThreads / kTileX, M = kTileZ / kLevels;
+    const int dx = threadIdx.x % kTileX, dz = threadIdx.x / kTileX, x = x0 + dx;
+    const B *src = b + (size_t)k * g.plane + ((size_t)(z0 + dz) * g.ny + y) * g.pitch + x;
+    B v[M];
+#pragma unroll
+    for (int j = 0; j < M; ++j)
+      if (x < g.nx && z0 + dz + j * kLevels < g.nz) v[j] = __ldg(src + (size_t)j * kLevels * g.ny * g.pitch);
+#pragma unroll
+    for (int j = 0; j < M; ++j) t[dx][dz + j * kLevels] = conv(v[j]);
   }
   __syncthreads();
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {   // r: x offset, threadIdx.x: z offset
-    const int x = x0 + r, z = z0 + threadIdx.x;
-    if (x < g.nx && z < g.nz) a[k * aplane + ((size_t)x * g.ny + y) * g.nz + z] = t[threadIdx.x][r];
-  }
-  (void)nk;
+  constexpr int kRows = kTileThreads / kTileZ, N = kTileX / kRows;
+  const int dz = threadIdx.x % kTileZ, dx = threadIdx.x / kTileZ, z = z0 + dz;
+  if (z >= g.nz) return;
+  A *dst = a + (size_t)k * g.nx * g.ny * g.nz + ((size_t)(x0 + dx) * g.ny + y) * g.nz + z;
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+    if (x0 + dx + j * kRows < g.nx) dst[(size_t)j * kRows * g.ny * g.nz] = t[dx + j * kRows][dz];
 }
 
-// Converters between a reference-layout value and the stored value of population k.
+// The weight of population k, as W<R>(k).
+template <typename R> __device__ __forceinline__ R weight_of(int k) {
+  return k == 0 ? W<R>(0) : k < 7 ? W<R>(1) : W<R>(7);
+}
+// Converters between a reference-layout value and the stored value of population k,
+// made once per block (Store::enc and Store::dec with the weight at run time).
 template <int DT, typename A> struct EncF {
-  __device__ typename Store<DT>::T operator()(int k, A v) const { return enc_dyn(k, (typename Store<DT>::R)v); }
-  __device__ typename Store<DT>::T pad(int k) const { return enc_dyn(k, W<typename Store<DT>::R>(k)); }
-  static __device__ typename Store<DT>::T enc_dyn(int k, typename Store<DT>::R v) {
-    typename Store<DT>::T out{};
-    static_for<0, Q>([&](auto I) {
-      constexpr int i = decltype(I)::value;
-      if (k == i) out = Store<DT>::template enc<i>(v);
-    });
-    return out;
-  }
+  using S = Store<DT>;
+  struct Of {
+    typename S::R w;
+    __device__ typename S::T operator()(A v) const {
+      if constexpr (S::kShift) return S::from_shifted((typename S::R)v - w);
+      else return (typename S::R)v;
+    }
+    __device__ typename S::T pad() const {
+      if constexpr (S::kShift) return S::from_shifted(w - w);
+      else return w;
+    }
+  };
+  __device__ Of operator()(int k) const { return {weight_of<typename S::R>(k)}; }
 };
 template <int DT, typename A> struct DecF {
-  __device__ A operator()(int k, typename Store<DT>::T v) const {
-    A out{};
-    static_for<0, Q>([&](auto I) {
-      constexpr int i = decltype(I)::value;
-      if (k == i) out = (A)Store<DT>::template dec<i>(v);
-    });
-    return out;
-  }
+  using S = Store<DT>;
+  struct Of {
+    typename S::R w;
+    __device__ A operator()(typename S::T v) const {
+      if constexpr (S::kShift) return (A)(w + S::to_shifted(v));
+      else return (A)v;
+    }
+  };
+  __device__ Of operator()(int k) const { return {weight_of<typename S::R>(k)}; }
 };
 template <typename A> struct Ident {
-  __device__ A operator()(int, A v) const { return v; }
-  __device__ A pad(int) const { return A(0); }
+  struct Of {
+    __device__ A operator()(A v) const { return v; }
+    __device__ A pad() const { return A(0); }
+  };
+  __device__ Of operator()(int) const { return {}; }
 };
 
 inline dim3 tgrid(const Geom &g, int nk, int xext) {
-  return dim3((unsigned)(nk * g.ny), (unsigned)((xext + 31) / 32), (unsigned)((g.nz + 31) / 32));
+  return dim3((unsigned)(nk * g.ny), (unsigned)((xext + kTileX - 1) / kTileX), (unsigned)((g.nz + kTileZ - 1) / kTileZ));
 }
 
 template <int DT>
 cudaError_t pack_f_t(const Geom &g, int ref_dtype, const void *ref, void *f, cudaStream_t s) {
   using T = typename Store<DT>::T;
   if (ref_dtype == SW_F32)
-    k_ref_to_dev<<<tgrid(g, Q, g.pitch), dim3(32, 8), 0, s>>>(g, Q, (const float *)ref, (T *)f, EncF<DT, float>{});
+    k_ref_to_dev<<<tgrid(g, Q, g.pitch), kTileThreads, 0, s>>>(g, (const float *)ref, (T *)f, EncF<DT, float>{});
   else
-    k_ref_to_dev<<<tgrid(g, Q, g.pitch), dim3(32, 8), 0, s>>>(g, Q, (const double *)ref, (T *)f, EncF<DT, double>{});
+    k_ref_to_dev<<<tgrid(g, Q, g.pitch), kTileThreads, 0, s>>>(g, (const double *)ref, (T *)f, EncF<DT, double>{});
   return cudaGetLastError();
 }
 template <int DT>
 cudaError_t unpack_f_t(const Geom &g, int ref_dtype, const void *f, void *ref, cudaStream_t s) {
   using T = typename Store<DT>::T;
   if (ref_dtype == SW_F32)
-    k_dev_to_ref<<<tgrid(g, Q, g.nx), dim3(32, 8), 0, s>>>(g, Q, (const T *)f, (float *)ref, DecF<DT, float>{});
+    k_dev_to_ref<<<tgrid(g, Q, g.nx), kTileThreads, 0, s>>>(g, (const T *)f, (float *)ref, DecF<DT, float>{});
   else
-    k_dev_to_ref<<<tgrid(g, Q, g.nx), dim3(32, 8), 0, s>>>(g, Q, (const T *)f, (double *)ref, DecF<DT, double>{});
+    k_dev_to_ref<<<tgrid(g, Q, g.nx), kTileThreads, 0, s>>>(g, (const T *)f, (double *)ref, DecF<DT, double>{});
   return cudaGetLastError();
 }
 
@@ -383,15 +414,15 @@ cudaError_t aux_unpack_f(const Geom &g, int dtype, int ref_dtype, const void *f,
   SW_DISPATCH(dtype, unpack_f_t<DT>(g, ref_dtype, f, ref, s));
 }
 cudaError_t aux_pack_flag(const Geom &g, const uint8_t *ref, uint8_t *flag, cudaStream_t s) {
-  k_ref_to_dev<<<tgrid(g, 1, g.pitch), dim3(32, 8), 0, s>>>(g, 1, ref, flag, Ident<uint8_t>{});
+  k_ref_to_dev<<<tgrid(g, 1, g.pitch), kTileThreads, 0, s>>>(g, ref, flag, Ident<uint8_t>{});
   return cudaGetLastError();
 }
 cudaError_t aux_unpack_u(const Geom &g, const float *u, float *ref, cudaStream_t s) {
-  k_dev_to_ref<<<tgrid(g, 4, g.nx), dim3(32, 8), 0, s>>>(g, 4, u, ref, Ident<float>{});
+  k_dev_to_ref<<<tgrid(g, 4, g.nx), kTileThreads, 0, s>>>(g, u, ref, Ident<float>{});
   return cudaGetLastError();
 }
 cudaError_t aux_unpack_acc(const Geom &g, const double *acc, double *ref, cudaStream_t s) {
-  k_dev_to_ref<<<tgrid(g, 4, g.nx), dim3(32, 8), 0, s>>>(g, 4, acc, ref, Ident<double>{});
+  k_dev_to_ref<<<tgrid(g, 4, g.nx), kTileThreads, 0, s>>>(g, acc, ref, Ident<double>{});
   return cudaGetLastError();
 }
 cudaError_t aux_build_tiles(const Geom &g, const uint8_t *flag, uint8_t *tiles, cudaStream_t s) {
