@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
 // copies issued at the start, bounded waits).  Odd step: the boxes are the
 // two-lattice step's (natural planes at the source rows and levels); interior
 // warps pull from them and scatter with aa_pair_collide_scatter, the others with
-// aa_odd_pair_edge.  Even step: box i is plane opp(i) -- slot i -- at
+// aa_odd_pair_edge.  Even step: one copy of all planes (slot i is plane opp(i)) at
 // the item's own rows and level; every warp collides from it as
 // aa_pair_even_fast does, warps next to stones or the ground with the link
 // masks of their cells (the stone links' force, cells that are not fluid left
@@ -496,15 +496,13 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
 // rest of a box (columns and rows of neighbouring items) may be read while
 // its owners rewrite it, and is not used.
 
-// Even step: the 19 own-slot boxes of item (x0, y0, z) and with ACC its sums.
+// Even step: the item's own slots in one copy of all planes (slot i is plane
+// opp(i): box OPP(i) of the stage) and with ACC its sums.
 template <bool ACC>
 __device__ __forceinline__ void tma_issue_own(const CUtensorMap *map, const CUtensorMap *map_acc, int x0, int y0, int z,
                                               uint32_t st, uint32_t bar) {
   mbar_expect_tx(bar, Q * kTmaBoxBytes + (ACC ? kTmaAccBytes : 0));
-  static_for<0, Q>([&](auto I) {
-    constexpr int i = decltype(I)::value;
-    tma_load_4d(st + i * kTmaBoxBytes, map, x0 - 8, y0, z, OPP(i), bar, Hold<false>{});
-  });
+  tma_load_4d(st, map, x0 - 8, y0, z, 0, bar, Hold<false>{});
   if constexpr (ACC) tma_load_4d(st + kTmaStageBytes, map_acc, x0, y0, z, 0, bar, Hold<false>{});
 }
 
@@ -552,7 +550,7 @@ __device__ __forceinline__ void aa_odd_pair_edge(const StepParams &p, const uint
   static_for<0, Q>([&](auto I) {
     constexpr int i = decltype(I)::value;
     constexpr int ex = CX(i), ey = CY(i);
-    const uint8_t *rowp = smem + i * kTmaBoxBytes + w * kTmaRowBytes;
+    const uint8_t *rowp = smem + box_slot(i) * kTmaBoxBytes + w * kTmaRowBytes;
     if constexpr (ey == 1) {
       if (y == 0) rowp = smem + Q * kTmaBoxBytes + wrap_slot(i) * kTmaWrapBytes;
     } else if constexpr (ey == -1) {
@@ -659,7 +657,7 @@ __device__ __forceinline__ void aa_odd_pair_checked(const StepParams &p, const u
   static_for<0, Q>([&](auto I) {
     constexpr int i = decltype(I)::value;
     constexpr int ex = CX(i), ey = CY(i);
-    const uint8_t *rowp = smem + i * kTmaBoxBytes + w * kTmaRowBytes;
+    const uint8_t *rowp = smem + box_slot(i) * kTmaBoxBytes + w * kTmaRowBytes;
     if constexpr (ey == 1) {
       if (y == 0) rowp = smem + Q * kTmaBoxBytes + wrap_slot(i) * kTmaWrapBytes;
     } else if constexpr (ey == -1) {
@@ -739,8 +737,8 @@ __device__ __forceinline__ void aa_odd_pair_checked(const StepParams &p, const u
 
 template <int DT, bool ODD, bool ACC, bool KEEP>
 __global__ void __launch_bounds__(128, 9)
-    k_step_aa_tma(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap map1,
-                  const __grid_constant__ CUtensorMap map_acc, const __grid_constant__ StepParams p, AAParams a) {
+    k_step_aa_tma(const __grid_constant__ LatticeMaps maps, const __grid_constant__ CUtensorMap map_acc,
+                  const __grid_constant__ StepParams p, AAParams a) {
   using PK = Pack16<DT>;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   __shared__ __align__(8) unsigned long long bar;
@@ -755,8 +753,8 @@ __global__ void __launch_bounds__(128, 9)
     mbar_init(smem_u32(&bar), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    if (ODD) tma_issue<ACC>(&map, &map1, &map_acc, g, x0s, y0, z, st, smem_u32(&bar));
-    else tma_issue_own<ACC>(&map, &map_acc, x0s, y0, z, st, smem_u32(&bar));
+    if (ODD) tma_issue<ACC>(maps, &map_acc, g, x0s, y0, z, st, smem_u32(&bar));
+    else tma_issue_own<ACC>(&maps.one, &map_acc, x0s, y0, z, st, smem_u32(&bar));
   }
   const int sa = 2 * bx;
   uint8_t ka = TILE_ALL_SOLID, kb = TILE_ALL_SOLID;
@@ -803,7 +801,8 @@ __global__ void __launch_bounds__(128, 9)
           f2 v[Q];
           static_for<0, Q>([&](auto I) {
             constexpr int i = decltype(I)::value;
-            v[i].v = PK::both(reinterpret_cast<const uint32_t *>(smem + i * kTmaBoxBytes + w * kTmaRowBytes)[lane_word]);
+            v[i].v = PK::both(
+                reinterpret_cast<const uint32_t *>(smem + OPP(i) * kTmaBoxBytes + w * kTmaRowBytes)[lane_word]);
           });
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
@@ -833,7 +832,8 @@ __global__ void __launch_bounds__(128, 9)
           f2 v[Q];
           static_for<0, Q>([&](auto I) {
             constexpr int i = decltype(I)::value;
-            v[i].v = PK::both(reinterpret_cast<const uint32_t *>(smem + i * kTmaBoxBytes + w * kTmaRowBytes)[lane_word]);
+            v[i].v = PK::both(
+                reinterpret_cast<const uint32_t *>(smem + OPP(i) * kTmaBoxBytes + w * kTmaRowBytes)[lane_word]);
           });
           const double2 *acc_box = reinterpret_cast<const double2 *>(smem + kTmaStageBytes) + w * 32 + lane;
           pair_collide_store<DT, ACC, false, KEEP>(p, v, x0, c, z, x0 == 0, has_b, [&](int k) { return acc_box[k * 4 * 32]; });
@@ -851,7 +851,8 @@ __global__ void __launch_bounds__(128, 9)
         static_for<0, Q>([&](auto I) {
           constexpr int i = decltype(I)::value;
           constexpr int ex = CX(i);
-          const uint32_t *r = reinterpret_cast<const uint32_t *>(smem + i * kTmaBoxBytes + w * kTmaRowBytes);
+          const uint32_t *r =
+              reinterpret_cast<const uint32_t *>(smem + box_slot(i) * kTmaBoxBytes + w * kTmaRowBytes);
           const uint32_t own = r[lane_word];                          // cells x0, x0 + 1
           if constexpr (ex == 0) {
             v[i].v = PK::both(own);
@@ -891,19 +892,21 @@ template <int DT> inline bool hold_aa(const StepParams &p) {
 // when the tensor maps cannot be made (the caller then runs k_step_aa_pair).
 template <int DT, bool ODD, bool ACC>
 cudaError_t launch_aa_tma(const StepParams &p, const AAParams &a, cudaStream_t s) {
-  CUtensorMap map, map1, map_acc;
-  if (!encode_lattice_map(&map, p.fin, p.g, 4) || !encode_lattice_map(&map1, p.fin, p.g, 1))
+  LatticeMaps maps;
+  CUtensorMap map_acc;
+  // the even step's only copy takes all populations (in `one`)
+  if (ODD ? !encode_lattice_maps(&maps, p.fin, p.g) : !encode_lattice_map(&maps.one, p.fin, p.g, 4, Q))
     return cudaErrorNotSupported;
   if (ACC) {
     if (!encode_acc_map(&map_acc, p.acc, p.g)) return cudaErrorNotSupported;
   } else {
-    map_acc = map;                                                   // not read
+    map_acc = maps.one;                                              // not read
   }
   constexpr int smem = tma_stage_bytes<ACC>() + 128;
   static_assert(smem <= 48 * 1024, "one stage fits the default shared memory of a block");
   const dim3 grid((unsigned)((p.g.nseg_x + 1) / 2), (unsigned)((p.g.ny + 3) / 4), (unsigned)p.g.nz);
-  if (!ODD && hold_aa<DT>(p)) k_step_aa_tma<DT, ODD, ACC, !ODD><<<grid, dim3(32, 4), smem, s>>>(map, map1, map_acc, p, a);
-  else k_step_aa_tma<DT, ODD, ACC, false><<<grid, dim3(32, 4), smem, s>>>(map, map1, map_acc, p, a);
+  if (!ODD && hold_aa<DT>(p)) k_step_aa_tma<DT, ODD, ACC, !ODD><<<grid, dim3(32, 4), smem, s>>>(maps, map_acc, p, a);
+  else k_step_aa_tma<DT, ODD, ACC, false><<<grid, dim3(32, 4), smem, s>>>(maps, map_acc, p, a);
   return cudaGetLastError();
 }
 

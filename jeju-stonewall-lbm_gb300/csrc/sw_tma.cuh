@@ -59,6 +59,23 @@ __host__ __device__ constexpr int wrap_slot(int i) {
        : i == 17 ? 8 : i == 18 ? 9 : -1;
 }
 
+// Where population i's box lies in a stage (in boxes): populations with the same
+// source row and level that one copy can fetch -- consecutive ones, or three
+// apart -- are neighbours.
+__host__ __device__ constexpr int box_slot(int i) {
+  constexpr int order[Q] = {0, 1, 2, 3, 7, 10, 4, 8, 9, 5, 11, 14, 6, 12, 13, 15, 16, 17, 18};
+  for (int k = 0; k < Q; ++k)
+    if (order[k] == i) return k;
+  return -1;
+}
+
+// The lattice's tensor maps: boxes of 80 cells x 4 rows of one population, of one
+// row, and of several populations -- 0 to 2, two consecutive ones, and the second
+// and third of every third population from 1 or from 2 on (7 and 10, 11 and 14).
+struct LatticeMaps {
+  CUtensorMap one, row, three, two, from1, from2;
+};
+
 // blocks that gave up waiting (must stay 0); one counter per translation unit
 static __device__ unsigned int g_tma_timeouts;
 
@@ -118,10 +135,11 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map
 
 // Issue the copies of item (x0, y0, z) into stage `st`, arriving on `bar` (one
 // thread); with ACC also the item's float64 sums (map_acc) behind the boxes.
-// KEEP: the copies hold their lines in L2, as the stores do.
+// KEEP: the copies hold their lines in L2, as the stores do.  13 copies below the
+// top level instead of one per population: the one thread that issues them is what
+// the block waits for (800x160x160 241.6 -> 239.8 us, 640x128x128 123.5 -> 122.6).
 template <bool ACC, bool KEEP = false>
-__device__ __forceinline__ void tma_issue(const CUtensorMap *map, const CUtensorMap *map1, const CUtensorMap *map_acc,
-                                          const Geom &g, int x0, int y0, int z, uint32_t st, uint32_t bar) {
+__device__ __forceinline__ void tma_issue(const LatticeMaps &m, const CUtensorMap *map_acc, const Geom &g, int x0, int y0, int z, uint32_t st, uint32_t bar) {
   const Hold<KEEP> hold;
   const bool top = z == g.nz - 1;
   const bool wrap_lo = y0 == 0;                  // source row -1 of the first warp (c_y = +1)
@@ -135,11 +153,26 @@ __device__ __forceinline__ void tma_issue(const CUtensorMap *map, const CUtensor
     constexpr int ey = CY(i), ez = CZ(i);
     const int pop = (ez == -1 && top) ? MIRZ(i) : i;
     const int zl = (ez == -1 && top) ? z : z - ez;
-    tma_load_4d(st + i * kTmaBoxBytes, map, x0 - 8, y0 - ey, zl, pop, bar, hold);
+    const uint32_t dst = st + box_slot(i) * kTmaBoxBytes;
+    if constexpr (i == 0) {
+      tma_load_4d(dst, &m.three, x0 - 8, y0, z, 0, bar, hold);
+    } else if constexpr (i == 7) {
+      tma_load_4d(dst, &m.from1, x0 - 8, y0 - 1, z, 2, bar, hold);       // and 10
+    } else if constexpr (i == 8) {
+      tma_load_4d(dst, &m.two, x0 - 8, y0 + 1, z, 8, bar, hold);         // and 9
+    } else if constexpr (i == 11) {
+      tma_load_4d(dst, &m.from2, x0 - 8, y0, z - 1, 3, bar, hold);       // and 14
+    } else if constexpr (i == 12 || i == 13) {
+      if (top) tma_load_4d(dst, &m.one, x0 - 8, y0, zl, pop, bar, hold);   // (their mirrors are 14 and 11)
+      else if (i == 12) tma_load_4d(dst, &m.two, x0 - 8, y0, z + 1, 12, bar, hold);
+    } else if constexpr (i != 1 && i != 2 && i != 9 && i != 10 && i != 14) {
+      tma_load_4d(dst, &m.one, x0 - 8, y0 - ey, zl, pop, bar, hold);
+    }
     if constexpr (ey == 1) {
-      if (wrap_lo) tma_load_4d(st + Q * kTmaBoxBytes + wrap_slot(i) * kTmaWrapBytes, map1, x0 - 8, g.ny - 1, zl, pop, bar, hold);
+      if (wrap_lo)
+        tma_load_4d(st + Q * kTmaBoxBytes + wrap_slot(i) * kTmaWrapBytes, &m.row, x0 - 8, g.ny - 1, zl, pop, bar, hold);
     } else if constexpr (ey == -1) {
-      if (wrap_hi) tma_load_4d(st + Q * kTmaBoxBytes + wrap_slot(i) * kTmaWrapBytes, map1, x0 - 8, 0, zl, pop, bar, hold);
+      if (wrap_hi) tma_load_4d(st + Q * kTmaBoxBytes + wrap_slot(i) * kTmaWrapBytes, &m.row, x0 - 8, 0, zl, pop, bar, hold);
     }
   });
   if constexpr (ACC) tma_load_4d(st + kTmaStageBytes, map_acc, x0, y0, z, 0, bar, hold);
@@ -169,7 +202,7 @@ __device__ __forceinline__ void tma_pair_fast(const StepParams &p, const uint8_t
   static_for<0, Q>([&](auto I) {
     constexpr int i = decltype(I)::value;
     constexpr int ex = CX(i), ey = CY(i);
-    const uint8_t *rowp = st + i * kTmaBoxBytes + w * kTmaRowBytes;
+    const uint8_t *rowp = st + box_slot(i) * kTmaBoxBytes + w * kTmaRowBytes;
     if constexpr (ey == 1 && !INTERIOR) {
       if (y == 0) rowp = st + Q * kTmaBoxBytes + wrap_slot(i) * kTmaWrapBytes;
     } else if constexpr (ey == -1 && !INTERIOR) {
@@ -205,8 +238,8 @@ __device__ __forceinline__ void tma_pair_fast(const StepParams &p, const uint8_t
 // Grid: (ceil(pitch / 64), ceil(ceil(ny / 4) / ITEMS), nz); block = 4 warps, warp w = row y0 + w.
 template <int DT, bool ACC, typename Cfg, bool KEEP>
 __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
-    k_step_tma(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap map1,
-               const __grid_constant__ CUtensorMap map_acc, const __grid_constant__ StepParams p) {
+    k_step_tma(const __grid_constant__ LatticeMaps maps, const __grid_constant__ CUtensorMap map_acc,
+               const __grid_constant__ StepParams p) {
   constexpr int kStage = tma_stage_bytes<ACC>();
   // With no more items than stages every item's copies are issued at the start
   // and no stage is reused: warps then run their items without block barriers.
@@ -229,7 +262,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     for (int j = 0; j < Cfg::NSTAGE && j < n_items; ++j)
-      tma_issue<ACC, KEEP>(&map, &map1, &map_acc, g, x0s, (yb0 + j) * 4, z, base + j * kStage, smem_u32(&bars[j]));
+      tma_issue<ACC, KEEP>(maps, &map_acc, g, x0s, (yb0 + j) * 4, z, base + j * kStage, smem_u32(&bars[j]));
   }
   // The segment classes of this warp's rows in all its items, fetched once up
   // front (lane j: segment 2 bx of item j, lane ITEMS + j: segment 2 bx + 1),
@@ -276,7 +309,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
       ok = __syncthreads_and(ok);                                     // barrier frees stage s
       if (!ok) break;
       if (leader && j + Cfg::NSTAGE < n_items)
-        tma_issue<ACC, KEEP>(&map, &map1, &map_acc, g, x0s, (yb0 + j + Cfg::NSTAGE) * 4, z, st, smem_u32(&bars[s]));
+        tma_issue<ACC, KEEP>(maps, &map_acc, g, x0s, (yb0 + j + Cfg::NSTAGE) * 4, z, st, smem_u32(&bars[s]));
     }
   }
   if constexpr (!kRing) ok = __syncthreads_and(ok);                 // every item was issued at the start
@@ -305,17 +338,27 @@ inline PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
-// The lattice f (16-bit elements, [19][nz][ny][pitch]) as a 4-D tensor, boxes of 80 x rows x 1 x 1.
-inline bool encode_lattice_map(CUtensorMap *m, const void *f, const Geom &g, int rows) {
+// The lattice f (16-bit elements, [19][nz][ny][pitch]) as a 4-D tensor, boxes of 80 x rows x 1 x pops;
+// with `step`, of every step-th population from `first` on.
+inline bool encode_lattice_map(CUtensorMap *m, const void *f, const Geom &g, int rows, int pops = 1, int first = 0,
+                               int step = 1) {
   auto enc = tensor_map_encoder();
   if (!enc) return false;
-  const cuuint64_t dim[4] = {(cuuint64_t)g.pitch, (cuuint64_t)g.ny, (cuuint64_t)g.nz, (cuuint64_t)Q};
-  const cuuint64_t stride[3] = {(cuuint64_t)g.pitch * 2, (cuuint64_t)g.pitch * g.ny * 2, (cuuint64_t)g.plane * 2};
-  const cuuint32_t box[4] = {(cuuint32_t)kTmaBoxX, (cuuint32_t)rows, 1, 1};
+  const cuuint64_t dim[4] = {(cuuint64_t)g.pitch, (cuuint64_t)g.ny, (cuuint64_t)g.nz,
+                             (cuuint64_t)((Q - first + step - 1) / step)};
+  const cuuint64_t stride[3] = {(cuuint64_t)g.pitch * 2, (cuuint64_t)g.pitch * g.ny * 2, (cuuint64_t)g.plane * 2 * step};
+  const cuuint32_t box[4] = {(cuuint32_t)kTmaBoxX, (cuuint32_t)rows, 1, (cuuint32_t)pops};
+  f = static_cast<const char *>(f) + (size_t)g.plane * 2 * first;
   const cuuint32_t estride[4] = {1, 1, 1, 1};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT16, 4, const_cast<void *>(f), dim, stride, box, estride,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+inline bool encode_lattice_maps(LatticeMaps *m, const void *f, const Geom &g) {
+  return encode_lattice_map(&m->one, f, g, 4) && encode_lattice_map(&m->row, f, g, 1) &&
+         encode_lattice_map(&m->three, f, g, 4, 3) && encode_lattice_map(&m->two, f, g, 4, 2) &&
+         encode_lattice_map(&m->from1, f, g, 4, 2, 1, 3) && encode_lattice_map(&m->from2, f, g, 4, 2, 2, 3);
 }
 
 // The float64 sums acc ([4][nz][ny][pitch]) as a 4-D tensor, boxes of 64 cells x 4 rows x 1 level x 4 sums.
@@ -340,13 +383,13 @@ inline bool hold_pair16(const Geom &g) { return g.plane * (2ll * Q * 2) > 118000
 
 template <int DT, bool ACC, typename Cfg, bool KEEP>
 cudaError_t launch_tma_as(const StepParams &p, cudaStream_t s) {
-  CUtensorMap map, map1, map_acc;
-  if (!encode_lattice_map(&map, p.fin, p.g, 4) || !encode_lattice_map(&map1, p.fin, p.g, 1))
-    return cudaErrorNotSupported;
+  LatticeMaps maps;
+  CUtensorMap map_acc;
+  if (!encode_lattice_maps(&maps, p.fin, p.g)) return cudaErrorNotSupported;
   if (ACC) {
     if (!encode_acc_map(&map_acc, p.acc, p.g)) return cudaErrorNotSupported;
   } else {
-    map_acc = map;                                                   // not read
+    map_acc = maps.one;                                              // not read
   }
   constexpr int smem = Cfg::NSTAGE * tma_stage_bytes<ACC>() + 128;   // + alignment slack
   static_assert(smem <= 227 * 1024, "stages exceed the shared memory of a block");
@@ -361,7 +404,7 @@ cudaError_t launch_tma_as(const StepParams &p, cudaStream_t s) {
   }
   const int nyb = (p.g.ny + 3) / 4;
   const dim3 grid((unsigned)((p.g.nseg_x + 1) / 2), (unsigned)((nyb + Cfg::ITEMS - 1) / Cfg::ITEMS), (unsigned)p.g.nz);
-  k_step_tma<DT, ACC, Cfg, KEEP><<<grid, dim3(32, 4), smem, s>>>(map, map1, map_acc, p);
+  k_step_tma<DT, ACC, Cfg, KEEP><<<grid, dim3(32, 4), smem, s>>>(maps, map_acc, p);
   return cudaGetLastError();
 }
 
