@@ -33,6 +33,8 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <type_traits>
+
 namespace sw {
 
 template <int ITEMS_, int NSTAGE_, int MINB_> struct TmaCfg {
@@ -69,12 +71,17 @@ __host__ __device__ constexpr int box_slot(int i) {
   return -1;
 }
 
-// The lattice's tensor maps: boxes of 80 cells x 4 rows of one population, of one
-// row, and of several populations -- 0 to 2, two consecutive ones, and the second
+// The lattice's tensor maps: boxes of 80 cells x 4 rows of one population and of one
+// row; and of several populations -- 0 to 2, two consecutive ones, and the second
 // and third of every third population from 1 or from 2 on (7 and 10, 11 and 14).
-struct LatticeMaps {
-  CUtensorMap one, row, three, two, from1, from2;
+struct SingleMaps {
+  CUtensorMap one, row;
 };
+struct LatticeMaps : SingleMaps {
+  CUtensorMap three, two, from1, from2;
+};
+// those of a two-lattice step: grouped copies where it holds lines (hold_pair16)
+template <bool KEEP> using StepMapsOf = std::conditional_t<KEEP, LatticeMaps, SingleMaps>;
 
 // blocks that gave up waiting (must stay 0); one counter per translation unit
 static __device__ unsigned int g_tma_timeouts;
@@ -135,11 +142,17 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map
 
 // Issue the copies of item (x0, y0, z) into stage `st`, arriving on `bar` (one
 // thread); with ACC also the item's float64 sums (map_acc) behind the boxes.
-// KEEP: the copies hold their lines in L2, as the stores do.  13 copies below the
-// top level instead of one per population: the one thread that issues them is what
-// the block waits for (800x160x160 241.6 -> 239.8 us, 640x128x128 123.5 -> 122.6).
-template <bool ACC, bool KEEP = false>
-__device__ __forceinline__ void tma_issue(const LatticeMaps &m, const CUtensorMap *map_acc, const Geom &g, int x0, int y0, int z, uint32_t st, uint32_t bar) {
+// KEEP: the copies hold their lines in L2, as the stores do.  With LatticeMaps 13
+// copies below the top level instead of one per population: the one thread that issues
+// them is what the block waits for (800x160x160 241.6 -> 239.8 us, 640x128x128 123.5 ->
+// 122.6).  Small lattices take SingleMaps: there four maps less to encode and to pass
+// (512 bytes of launch parameters) count as much, and walls side by side in one graph
+// lost by the grouped copies (us per step, one copy per population / grouped: eight
+// walls of H 10 to 24 83.4 / 87.0, three of H 9 to 21 21.8 / 22.7).
+template <bool ACC, bool KEEP = false, typename Maps>
+__device__ __forceinline__ void tma_issue(const Maps &m, const CUtensorMap *map_acc, const Geom &g, int x0, int y0,
+                                          int z, uint32_t st, uint32_t bar) {
+  constexpr bool kGrouped = std::is_same<Maps, LatticeMaps>::value;
   const Hold<KEEP> hold;
   const bool top = z == g.nz - 1;
   const bool wrap_lo = y0 == 0;                  // source row -1 of the first warp (c_y = +1)
@@ -154,7 +167,9 @@ __device__ __forceinline__ void tma_issue(const LatticeMaps &m, const CUtensorMa
     const int pop = (ez == -1 && top) ? MIRZ(i) : i;
     const int zl = (ez == -1 && top) ? z : z - ez;
     const uint32_t dst = st + box_slot(i) * kTmaBoxBytes;
-    if constexpr (i == 0) {
+    if constexpr (!kGrouped) {
+      tma_load_4d(dst, &m.one, x0 - 8, y0 - ey, zl, pop, bar, hold);
+    } else if constexpr (i == 0) {
       tma_load_4d(dst, &m.three, x0 - 8, y0, z, 0, bar, hold);
     } else if constexpr (i == 7) {
       tma_load_4d(dst, &m.from1, x0 - 8, y0 - 1, z, 2, bar, hold);       // and 10
@@ -238,7 +253,7 @@ __device__ __forceinline__ void tma_pair_fast(const StepParams &p, const uint8_t
 // Grid: (ceil(pitch / 64), ceil(ceil(ny / 4) / ITEMS), nz); block = 4 warps, warp w = row y0 + w.
 template <int DT, bool ACC, typename Cfg, bool KEEP>
 __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
-    k_step_tma(const __grid_constant__ LatticeMaps maps, const __grid_constant__ CUtensorMap map_acc,
+    k_step_tma(const __grid_constant__ StepMapsOf<KEEP> maps, const __grid_constant__ CUtensorMap map_acc,
                const __grid_constant__ StepParams p) {
   constexpr int kStage = tma_stage_bytes<ACC>();
   // With no more items than stages every item's copies are issued at the start
@@ -355,8 +370,12 @@ inline bool encode_lattice_map(CUtensorMap *m, const void *f, const Geom &g, int
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+inline bool encode_lattice_maps(SingleMaps *m, const void *f, const Geom &g) {
+  return encode_lattice_map(&m->one, f, g, 4) && encode_lattice_map(&m->row, f, g, 1);
+}
+
 inline bool encode_lattice_maps(LatticeMaps *m, const void *f, const Geom &g) {
-  return encode_lattice_map(&m->one, f, g, 4) && encode_lattice_map(&m->row, f, g, 1) &&
+  return encode_lattice_maps(static_cast<SingleMaps *>(m), f, g) &&
          encode_lattice_map(&m->three, f, g, 4, 3) && encode_lattice_map(&m->two, f, g, 4, 2) &&
          encode_lattice_map(&m->from1, f, g, 4, 2, 1, 3) && encode_lattice_map(&m->from2, f, g, 4, 2, 2, 3);
 }
@@ -374,16 +393,19 @@ inline bool encode_acc_map(CUtensorMap *m, const double *acc, const Geom &g) {
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Whether a 16-bit two-lattice step holds lines in L2: once the lattice pair
-// exceeds the L2 (us per step, streaming / held: 280x56x56, 67 MB a pair, 13.0 /
+// Whether a 16-bit two-lattice step holds lines in L2 (and groups its copies): once the
+// lattice pair exceeds the L2 (us per step, streaming / held: 280x56x56, 67 MB a pair, 13.0 /
 // 13.5; 320x64x64, 100 MB, 17.8 / 18.0; 352x68x68, 124 MB, 26.1 / 25.8; 360x72x72,
 // 145 MB, 29.7 / 28.8; 440x88x88 48.0 / 46.2; 800x160x160 245 / 243, accumulating
-// 281 / 278).
+// 281 / 278).  The line holds for walls side by side in one graph too (us per step, all
+// streaming / by this rule: six of H 19 208.0 / 206.3, four of H 22 210.1 / 205.4, three
+// of H 32 436.6 / 426.2, two of H 40 568.5 / 556.5); a mix of mostly smaller walls can
+// lose (H 8 to 27, two of the six above the line: 173.9 / 174.8).
 inline bool hold_pair16(const Geom &g) { return g.plane * (2ll * Q * 2) > 118000000ll; }
 
 template <int DT, bool ACC, typename Cfg, bool KEEP>
 cudaError_t launch_tma_as(const StepParams &p, cudaStream_t s) {
-  LatticeMaps maps;
+  StepMapsOf<KEEP> maps;
   CUtensorMap map_acc;
   if (!encode_lattice_maps(&maps, p.fin, p.g)) return cudaErrorNotSupported;
   if (ACC) {
