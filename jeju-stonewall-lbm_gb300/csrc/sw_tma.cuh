@@ -12,7 +12,8 @@
 // tensor-memory accelerator, which copies it into shared memory and signals an
 // mbarrier.  Warps then read their two cells' sources from the box row at the
 // shifted offset (two aligned 32-bit shared loads and a byte permute for
-// c_x = +-1, one load otherwise).
+// c_x = +-1, one load otherwise).  On large lattices one copy fetches the boxes of
+// populations with the same source row and level (box_slot, tma_issue).
 //
 // Boxes start on 16-byte boundaries (x0 - 8 is a multiple of 8 halves); a box
 // reaching outside the lattice reads zeros there: x < 0 only feeds the inlet
