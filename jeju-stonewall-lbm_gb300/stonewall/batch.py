@@ -292,23 +292,24 @@ class Batch:
         return sum(m.grid.cells for m in self.members)
 
     def autotune(self, repeats=5, modes=("persistent", "graph")):
-        """Time the persistent kernel in every configuration this storage type has, and the graph
-        mode (with the single-lattice configurations tuned on the largest member), on the current
-        members; keep the fastest.  Each timed step recomputes every member's next state into its
-        spare buffer with forces and sums switched off, so the members' states are not changed.
+        """Time the persistent kernel in every configuration that gives this storage type's bits
+        (autotune.candidates), and the graph mode (with the single-lattice configurations tuned on
+        the largest member), on the current members; keep the fastest.  Each timed step recomputes
+        every member's next state into its spare buffer with forces and sums switched off, so the
+        members' states are not changed.
         Returns (best, times): best is a configuration number or "graph"."""
+        from . import autotune as single
         times = {}
         if any(getattr(m, "pattern", "ab") == "aa" for m in self.members):
             # in-place members: graph mode, and no trial steps (they would change those states); the
             # two-lattice members' configurations are still tuned on the largest of them
             ab = [m for m in self.pending() if getattr(m, "pattern", "ab") == "ab"]
             if ab:
-                from . import autotune as single
                 single.tune(max(ab, key=lambda m: m.grid.cells))
             self.mode = "graph"
             return "graph", times
         if "persistent" in modes:
-            for cfg in range(N.lib().sw_step_config_count()):
+            for cfg in single.candidates(self.dtype):
                 if not _valid(self.dtype, cfg):
                     continue
                 self.cfg = cfg
@@ -325,7 +326,6 @@ class Batch:
             self.cfg = min(times, key=times.get)
         live = self.pending()
         if "graph" in modes and 0 < len(live) <= GRAPH_MAX:
-            from . import autotune as single
             single.tune(max(live, key=lambda m: m.grid.cells))
             slot, lv = self._fill(1, tuning=True, upload=False)
             self._graph_run(slot, len(lv), 1)                       # instantiate
