@@ -118,7 +118,8 @@ __host__ __device__ __forceinline__ double of_units(u64 v) {
   return of_bits(join(hi32(r) + ((1023u - s) << 20), lo32(r)));   // v = 2^(63 - s) 1.f units: exponent 1 - s
 }
 
-// A double in [1/4, 4) as a whole number of units, exact (2^-62 divides its last place).
+// A double in [1/4, 4) as a whole number of units, exact (2^-62 divides its last place); from 2 on the bits are
+// those of an unsigned number.
 __host__ __device__ __forceinline__ i64 to_units_large(double v) {
   const u64 b = bits_of(v);
   const uint32_t t = (hi32(b) >> 20) - kExpMin, m = (hi32(b) & 0xfffffu) | 0x100000u;
@@ -177,7 +178,8 @@ __host__ __device__ __forceinline__ bool collide(const double (&f)[19], double t
   const i64 mz = d[2] + (d[5] - d[6]) + (d[7] - d[8]);
   mom.rho = of_units((u64)rho);
   const double y = reciprocal(mom.rho);
-  const i64 inv = to_units_large(y);                // 1 / rho in (1/2, 2]
+  const i64 inv = to_units_large(y);                // 1 / rho in (1/2, 2)
+  if (inv < 0) return false;                        // a density that rounds to 1/2: its reciprocal 2 has no sign bit left
   // |m| < 3/4, |u| < 3/2: u and m u in units of 2^-61
   const i64 ux = mom.u[0] = mulhi(mx << 1, inv), uy = mom.u[1] = mulhi(my << 1, inv), uz = mom.u[2] = mulhi(mz << 1, inv);
   const i64 mx2 = mx << 1, my2 = my << 1, mz2 = mz << 1, ux2 = ux << 1, uy2 = uy << 1, uz2 = uz << 1;
