@@ -205,9 +205,10 @@ __host__ __device__ __forceinline__ bool collide(const double (&f)[19], double t
   const uint32_t qh = hi32((u64)q) < 256u ? 256u : hi32((u64)q);
   const double qn = scaled(square_root(of_units(join(qh, lo32((u64)q)))), 1 - lead);
   const double root = square_root(dfma(dmul(c18, y), qn, tau0sq));
-  // keep = 1 - 1 / tau, tau = (tau0 + root) / 2 > 1/2; tau of 4 and above is left to double
+  // keep = 1 - 1 / tau, tau = (tau0 + root) / 2; a 1 / tau outside [1/4, 2 + 2^-19), negative, infinite or NaN (one
+  // unsigned range of the upper word) is left to double
   const double rt = scaled(reciprocal(dadd(tau0, root)), 1);
-  if (hi32(bits_of(rt)) < (1021u << 20)) return false;
+  if (hi32(bits_of(rt)) - (1021u << 20) > (3u << 20)) return false;
   const i64 keep = (i64)((1ull << 62) - (u64)to_units_large(rt));
   const i64 Bxx = bxx + mulhi(nxx << 1, keep), Byy = byy + mulhi(nyy << 1, keep), Bzz = bzz + mulhi(nzz << 1, keep);
   const i64 Bxy = bxy + mulhi(nxy << 1, keep), Bxz = bxz + mulhi(nxz << 1, keep), Byz = byz + mulhi(nyz << 1, keep);
