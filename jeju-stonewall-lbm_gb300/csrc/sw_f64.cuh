@@ -149,12 +149,13 @@ __host__ __device__ __forceinline__ double square_root(double v) {
 }
 
 // The collision of one cell.  tau0 = 3 nu + 1/2, tau0sq its square, c18 = 18 sqrt(2) Cs^2.  out[i] receives the
-// new populations and mom rho and u (those are formed where they are used); false: the cell is out of range and
-// nothing of it is valid.
+// new populations and mom rho and u (those are formed where they are used: from the exact m, so that velocities
+// near rest keep their relative precision, which the collision's own u in units of 2^-61 has not); false: the
+// cell is out of range and nothing of it is valid.
 struct Moments {
-  double rho;
-  i64 u[3];                                         // u in units of 2^-61
-  __host__ __device__ __forceinline__ double vel(int k) const { return dmul(of_int(u[k]), 1.0 / 2305843009213693952.0); }
+  double rho, inv;                                  // inv: 2^-62 / rho
+  i64 m[3];                                         // m in units of 2^-62
+  __host__ __device__ __forceinline__ double vel(int k) const { return dmul(of_int(m[k]), inv); }
 };
 __host__ __device__ __forceinline__ bool collide(const double (&f)[19], double tau0, double tau0sq, double c18,
                                                  double (&out)[19], Moments &mom) {
@@ -178,10 +179,12 @@ __host__ __device__ __forceinline__ bool collide(const double (&f)[19], double t
   const i64 mz = d[2] + (d[5] - d[6]) + (d[7] - d[8]);
   mom.rho = of_units((u64)rho);
   const double y = reciprocal(mom.rho);
+  mom.inv = scaled(y, -62);
+  mom.m[0] = mx, mom.m[1] = my, mom.m[2] = mz;
   const i64 inv = to_units_large(y);                // 1 / rho in (1/2, 2)
   if (inv < 0) return false;                        // a density that rounds to 1/2: its reciprocal 2 has no sign bit left
   // |m| < 3/4, |u| < 3/2: u and m u in units of 2^-61
-  const i64 ux = mom.u[0] = mulhi(mx << 1, inv), uy = mom.u[1] = mulhi(my << 1, inv), uz = mom.u[2] = mulhi(mz << 1, inv);
+  const i64 ux = mulhi(mx << 1, inv), uy = mulhi(my << 1, inv), uz = mulhi(mz << 1, inv);
   const i64 mx2 = mx << 1, my2 = my << 1, mz2 = mz << 1, ux2 = ux << 1, uy2 = uy << 1, uz2 = uz << 1;
   const i64 bxx = mulhi(mx2, ux2), byy = mulhi(my2, uy2), bzz = mulhi(mz2, uz2);
   const i64 bxy = mulhi(mx2, uy2), bxz = mulhi(mx2, uz2), byz = mulhi(my2, uz2);
