@@ -121,8 +121,9 @@ class Flags:
             raise ValueError(f"flag has shape {f.shape}, expected {(grid.nx, grid.ny, grid.nz)}")
         self.flag = torch.empty(grid.cells_padded, dtype=torch.uint8, device=device)
         self.tiles = torch.empty(grid.tiles, dtype=torch.uint8, device=device)
-        self._given = torch.empty((grid.nx, grid.ny, grid.nz), dtype=torch.uint8, device=device)
-        self._ref, self._host = self._given, None
+        self._ref = torch.empty((grid.nx, grid.ny, grid.nz), dtype=torch.uint8, device=device)
+        self._given = self._ref            # the construction's flags until `host` has them
+        self._host = self._solid = None
         self._upload(torch.from_numpy(f), stream)
         (stream or torch.cuda.current_stream()).synchronize()
 
@@ -130,8 +131,20 @@ class Flags:
     def host(self):
         """The flags given at construction (NumPy, reference layout), downloaded when first asked for."""
         if self._host is None:
-            self._host = _download(self._given)
+            self._host, self._given = _download(self._given), None
         return self._host
+
+    def solid(self):
+        """Where the cells are not fluid now, after the last load() (NumPy, reference layout)."""
+        if self._solid is None:
+            self._solid = _download(self._ref) != 0
+        return self._solid
+
+    @property
+    def nbytes(self):
+        """Device bytes held."""
+        kept = self._given is not None and self._given is not self._ref
+        return self.flag.numel() + self.tiles.numel() + self._ref.numel() * (2 if kept else 1)
 
     def load(self, flag_ref, stream=None):
         """Copy flags (reference layout, host or device tensor; pinned host memory copies
@@ -141,6 +154,7 @@ class Flags:
             raise ValueError(f"flag must be uint8 {(g.nx, g.ny, g.nz)}")
         if self._ref is self._given:
             self._ref = torch.empty_like(self._given)           # the construction's flags stay for `host`
+        self._solid = None
         self._upload(flag_ref, stream)
 
     def _upload(self, flag_ref, stream):

@@ -132,7 +132,7 @@ def solve_stats_host(s):
     p = s.params
     co = coefficients(s.force_series(), p.UH, p.H, p.ny)
     st = stats(co["Cd"], co["Cm"], co["Cl"], s.n_spin)
-    wall = s.flags.numpy() != 0
+    wall = s.flags.solid()
     st["recirc"] = recirculation_area(s.mean_field()[1][::2, ::2, ::2], wall[::2, ::2, ::2], p.H, p.X0, p.UH, p.ny)
     return st
 

@@ -151,10 +151,8 @@ class WallSolver:
         return self.f[0].dtype
 
     def memory_bytes(self):
-        g = self.grid
-        return (sum(f.nbytes for f in self.f) + self.flags.flag.numel() + self.flags.tiles.numel()
-                + self.force.data.numel() * 8 + self.acc.data.numel() * 8
-                + (self.ghost.numel() if self.pattern == "aa" else 0))
+        return (sum(f.nbytes for f in self.f) + self.flags.nbytes + self.force.data.numel() * 8
+                + self.acc.data.numel() * 8 + (self.ghost.numel() if self.pattern == "aa" else 0))
 
     def reload(self, flag, uin):
         """Start over with a new mask and inlet profile (torch tensors, pinned host memory copies
@@ -343,7 +341,7 @@ class WallSolver:
 
     def sums(self):
         """Running sums of (rho, u), reference layout, solids at n_acc * (1, 0, 0, 0) (lbm3d.py:303)."""
-        return self.acc.numpy(solid=self.flags.host != 0, n_acc=self.n_acc)
+        return self.acc.numpy(solid=self.flags.solid(), n_acc=self.n_acc)
 
     def mean_field(self):
         """Time-mean (rho, u) over the accumulated states, float64 (lbm3d.py:402)."""
@@ -384,7 +382,7 @@ class WallSolver:
                 d.record_stream(side)
         copied = torch.cuda.Event()
         copied.record(side)
-        solid, n_acc, state = self.flags.host != 0, self.n_acc, dict(t=self.t, n_acc=self.n_acc, sig=sig)
+        solid, n_acc, state = self.flags.solid(), self.n_acc, dict(t=self.t, n_acc=self.n_acc, sig=sig)
         extra = dict(extra or {})
 
         def write():
