@@ -124,6 +124,7 @@ class Flags:
         self._ref = torch.empty((grid.nx, grid.ny, grid.nz), dtype=torch.uint8, device=device)
         self._given = self._ref            # the construction's flags until `host` has them
         self._host = self._solid = None
+        self.version = object()            # another one after each load()
         self._upload(torch.from_numpy(f), stream)
         (stream or torch.cuda.current_stream()).synchronize()
 
@@ -140,6 +141,14 @@ class Flags:
             self._solid = _download(self._ref) != 0
         return self._solid
 
+    def solid_if_known(self):
+        """solid() where that needs no download, else None."""
+        return self._solid
+
+    def ref_copy(self):
+        """A device copy of the flags after the last load(), in the reference layout."""
+        return self._ref.clone()
+
     @property
     def nbytes(self):
         """Device bytes held."""
@@ -154,7 +163,7 @@ class Flags:
             raise ValueError(f"flag must be uint8 {(g.nx, g.ny, g.nz)}")
         if self._ref is self._given:
             self._ref = torch.empty_like(self._given)           # the construction's flags stay for `host`
-        self._solid = None
+        self._solid, self.version = None, object()
         self._upload(flag_ref, stream)
 
     def _upload(self, flag_ref, stream):

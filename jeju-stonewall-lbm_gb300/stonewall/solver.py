@@ -125,7 +125,8 @@ class WallSolver:
         self._q_levels = (None, None)   # quantisation levels of q_frame on the device, for one qmax
         self._ring = None
         self.launches = 0          # kernels of this library launched by advance()
-        self._ckpt_host = None     # pinned host buffers of the checkpoint writer (reused)
+        self._ckpt_host = ()       # pinned host buffers of the checkpoint writer (reused)
+        self._ckpt_solid = (None, None)   # the mask the last checkpoint downloaded, and its version
         self._ckpt_stream = None
         self._ckpt_thread = None
         self._ckpt_error = None
@@ -366,28 +367,34 @@ class WallSolver:
         acc_dev = torch.empty((4, g.nx, g.ny, g.nz), dtype=torch.float64, device=self.device)
         N.check(N.lib().sw_unpack_acc(g.gp, self.acc.ptr, _ptr(acc_dev), _stream(main)), "sw_unpack_acc")
         force_dev = self.force.data.clone()
+        # the mask with the rest, unless the host has it: asking for it here would wait for the queued steps
+        version = self.flags.version
+        known = self._ckpt_solid[1] if self._ckpt_solid[0] is version else self.flags.solid_if_known()
+        parts = (f_dev, acc_dev, force_dev) + (() if known is not None else (self.flags.ref_copy(),))
         taken = torch.cuda.Event()
         taken.record(main)
-        host = self._ckpt_host
-        if host is None or host[0].shape != f_dev.shape or host[0].dtype != f_dev.dtype:
-            host = tuple(torch.empty(t.shape, dtype=t.dtype, pin_memory=True) for t in (f_dev, acc_dev, force_dev))
-            self._ckpt_host = host
+        old = self._ckpt_host
+        host = tuple(old[i] if i < len(old) and (old[i].shape, old[i].dtype) == (t.shape, t.dtype)
+                     else torch.empty(t.shape, dtype=t.dtype, pin_memory=True) for i, t in enumerate(parts))
+        self._ckpt_host = host + old[len(host):]
         if self._ckpt_stream is None:
             self._ckpt_stream = torch.cuda.Stream(device=self.device)
         side = self._ckpt_stream
         side.wait_event(taken)
         with torch.cuda.stream(side):
-            for h, d in zip(host, (f_dev, acc_dev, force_dev)):
+            for h, d in zip(host, parts):
                 h.copy_(d, non_blocking=True)
                 d.record_stream(side)
         copied = torch.cuda.Event()
         copied.record(side)
-        solid, n_acc, state = self.flags.solid(), self.n_acc, dict(t=self.t, n_acc=self.n_acc, sig=sig)
+        n_acc, state = self.n_acc, dict(t=self.t, n_acc=self.n_acc, sig=sig)
         extra = dict(extra or {})
 
         def write():
             copied.synchronize()
-            f_h, acc_h, force_h = (h.numpy() for h in host)
+            f_h, acc_h, force_h = (h.numpy() for h in host[:3])
+            solid = known if known is not None else host[3].numpy() != 0
+            self._ckpt_solid = (version, solid)                     # (read once this writer is joined)
             acc_h[0][solid] = float(n_acc)                          # what k_macro + k_accum give solids
             acc_h[1:, solid] = 0.0
             tmp = path + ".tmp"
