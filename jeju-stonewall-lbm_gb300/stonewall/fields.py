@@ -167,8 +167,17 @@ class Flags:
         self._upload(flag_ref, stream)
 
     def _upload(self, flag_ref, stream):
+        """All on the one stream: a given one also waits for what the current one has made of flag_ref."""
         g = self.grid
-        self._ref.copy_(flag_ref, non_blocking=True)
+        if stream is None:
+            self._ref.copy_(flag_ref, non_blocking=True)
+        else:
+            stream.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(stream):
+                self._ref.copy_(flag_ref, non_blocking=True)
+            for t in (flag_ref, self._ref, self.flag, self.tiles):
+                if t.is_cuda:
+                    t.record_stream(stream)
         s = _stream(stream)
         N.check(N.lib().sw_pack_flag(g.gp, _ptr(self._ref), _ptr(self.flag), s), "sw_pack_flag")
         N.check(N.lib().sw_build_tiles(g.gp, _ptr(self.flag), _ptr(self.tiles), s), "sw_build_tiles")
