@@ -114,7 +114,8 @@ class Flags:
 
     def __init__(self, grid, flag_ref, device="cuda", stream=None):
         self.grid = grid
-        f = np.ascontiguousarray(flag_ref, dtype=np.uint8)      # (the caller's array, if it is one already)
+        # (the caller's array, if it is one already; other values wrap, those of a nested list too)
+        f = np.ascontiguousarray(np.asarray(flag_ref).astype(np.uint8, copy=False))
         if not f.flags.writeable:                               # (torch takes writable arrays)
             f = f.copy()
         if f.shape != (grid.nx, grid.ny, grid.nz):
