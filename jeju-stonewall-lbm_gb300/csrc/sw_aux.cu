@@ -751,16 +751,18 @@ __global__ void __launch_bounds__(kQThreads) k_qcoarse(Geom g, const float *u, c
 }
 
 // The planes of a snapshot (lbm3d.py:371-375): ux, uy, uz at y = y0 as
-// [3][nx][nz], then at z = z0 as [3][nx][ny], rounded to half precision.
+// [3][nx][nz], then at z = z0 as [3][nx][ny], rounded to half precision.  One
+// component per blockIdx.y: a plane of one has fewer cells than 2^31, three may not.
 __global__ void k_snapshot(Geom g, const float *u, int y0, int z0, __half *out) {
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long xz = 3ll * g.nx * g.nz, xy = 3ll * g.nx * g.ny;
+  const long long xz = (long long)g.nx * g.nz, xy = (long long)g.nx * g.ny;
   if (e >= xz + xy) return;
   const bool side = e < xz;
-  const uint32_t r = (uint32_t)(side ? e : e - xz), n = (uint32_t)(side ? g.nz : g.ny);
-  const uint32_t cx = r / n, w = r - cx * n, c = cx / (uint32_t)g.nx, x = cx - c * (uint32_t)g.nx;
+  const uint32_t c = blockIdx.y, r = (uint32_t)(side ? e : e - xz), n = (uint32_t)(side ? g.nz : g.ny);
+  const uint32_t x = r / n, w = r - x * n;
   const size_t row = side ? (size_t)w * g.ny + y0 : (size_t)z0 * g.ny + w;
-  out[e] = __float2half_rn(u[(size_t)(c + 1) * g.plane + row * g.pitch + x]);
+  __half *plane = side ? out + c * xz : out + 3 * xz + c * xy;
+  plane[r] = __float2half_rn(u[(size_t)(c + 1) * g.plane + row * g.pitch + x]);
 }
 
 // The log quantisation of a Q frame (lbm3d.py:317-318) by its level boundaries:
@@ -799,8 +801,8 @@ cudaError_t aux_qcoarse(const Geom &g, const float *u, const uint8_t *flag, int 
   return cudaGetLastError();
 }
 cudaError_t aux_snapshot(const Geom &g, const float *u, int y0, int z0, void *out, cudaStream_t s) {
-  const long long n = 3ll * g.nx * ((long long)g.nz + g.ny);
-  k_snapshot<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(g, u, y0, z0, static_cast<__half *>(out));
+  const long long n = (long long)g.nx * ((long long)g.nz + g.ny);
+  k_snapshot<<<dim3((unsigned)((n + 255) / 256), 3), 256, 0, s>>>(g, u, y0, z0, static_cast<__half *>(out));
   return cudaGetLastError();
 }
 cudaError_t aux_quantise(const float *q, long long n, float scale, float qmax, const float *levels, uint8_t *out,

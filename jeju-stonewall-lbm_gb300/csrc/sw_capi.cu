@@ -473,7 +473,7 @@ int sw_qcoarse(const sw_geom *g, const float *u, const uint8_t *flag, int32_t x0
 
 int sw_snapshot_planes(const sw_geom *g, const float *u, int32_t y0, int32_t z0, void *out, sw_stream s) {
   if (!geom_ok(g) || !u || !out || y0 < 0 || y0 >= g->ny || z0 < 0 || z0 >= g->nz) return SW_ERR_BAD_ARG;
-  if (((uintptr_t)out & 1u) || 3ll * g->nx * std::max(g->ny, g->nz) >= (1ll << 32)) return SW_ERR_BAD_ARG;
+  if ((uintptr_t)out & 1u) return SW_ERR_BAD_ARG;
   clear_stale();
   return cuda_status(sw::aux_snapshot(to_geom(g), u, y0, z0, out, st(s)));
 }
