@@ -318,11 +318,11 @@ class WallSolver:
         # q is float32, so plain numbers scale and clip it in float32; others (a numpy float64 would
         # widen it) and limits without 255 levels below them stay with the expression itself
         if type(q_scale) in (int, float) and type(qmax) in (int, float) and 0 < q_scale < 1e30 and 1e-3 < qmax < 1e30:
-            key = float(qmax)
-            if self._q_levels[0] != key:
-                self._q_levels = (key, torch.from_numpy(quantise_levels(key)).to(self.device))
+            key, kept = float(qmax), self._q_levels     # (one read: another thread may ask for another limit)
+            if kept[0] != key:
+                kept = self._q_levels = (key, torch.from_numpy(quantise_levels(key)).to(self.device))
             out = torch.empty(tuple(dims), dtype=torch.uint8, device=self.device)
-            N.check(N.lib().sw_quantise_levels(_ptr(q), q.numel(), float(q_scale), key, _ptr(self._q_levels[1]),
+            N.check(N.lib().sw_quantise_levels(_ptr(q), q.numel(), float(q_scale), key, _ptr(kept[1]),
                                                _ptr(out), _stream(None)), "sw_quantise_levels")
             return out.cpu().numpy()
         return _quantise(np.clip(q.cpu().numpy() * q_scale, 0, qmax), qmax)
