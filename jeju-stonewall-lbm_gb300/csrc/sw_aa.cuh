@@ -875,17 +875,20 @@ __global__ void __launch_bounds__(128, 9)
   }
 }
 
-// Whether an in-place step holds lines in L2.  The 16-bit even step (whose stores
-// are whole words): lattices well above the L2 (us per step, streaming / held, odd
+// Whether an in-place step holds lines in L2 (129 MB).  The 16-bit even step (whose stores
+// are whole words): lattices well above it (us per step, streaming / held, odd
 // and even together: 480x96x96, 168 MB, 77.9 / 78.7; 520x104x104 94.2 / 93.2;
-// 640x128x128 157 / 152; 800x160x160 299 / 286).  float32: where the one lattice
-// fits the L2 (320x64x64 35.4 / 30.6) and from about 300 MB (800x160x160 498 /
-// 496); between them only the accumulating steps (420x84x84 plain 80.9 / 82.1,
-// accumulating 88.1 / 87.9).
+// 640x128x128 157 / 152; 800x160x160 299 / 286).  float32: accumulating steps, and
+// plain ones of a lattice that the L2 takes whole with its sums and flags beside it
+// (us per step of a solve that accumulates every fifth, plain steps streaming / held:
+// 240x48x48, 42 MB, 18.0 / 17.5; 280x56x56, 76 MB, 23.7 / 22.9; 320x64x64, 100 MB, 37.7 /
+// 37.5; 340x68x68, 124 MB, 49.7 / 52.5; 480x96x96 127 / 129; 720x144x144 415 / 416;
+// 800x160x160 551 / 551).  The held float32 form is compiled separately and other
+// multiply-adds are fused in it: across the line solves differ by rounding.
 template <int DT> inline bool hold_aa(const StepParams &p) {
   const long long bytes = p.g.plane * Q * (long long)sizeof(typename Store<DT>::T);
   if (is16(DT)) return bytes > 180000000ll;
-  return DT == SW_F32 && (p.acc != nullptr || bytes < 126000000ll || bytes > 300000000ll);
+  return DT == SW_F32 && (p.acc != nullptr || bytes < 112000000ll);
 }
 
 // The TMA-staged AA step on the lattice p.fin (== p.fout); cudaErrorNotSupported
