@@ -937,13 +937,15 @@ cudaError_t launch_aa(const StepParams &p_in, const AAParams &a, bool odd, cudaS
     if (e != cudaSuccess) return e;
   }
   if constexpr (is16(DT)) {                          // two cells per thread, sources staged by TMA
-    if (a.tma) {
+    // Not the odd step of a grid one cell long: its inlet cells are its outlet cells, and the
+    // targets in their own column need not be fluid, which only the per-cell code looks at.
+    if (a.tma && !(odd && p.g.nx == 1)) {
       cudaError_t e = odd ? (p.acc ? launch_aa_tma<DT, true, true>(p, a, s) : launch_aa_tma<DT, true, false>(p, a, s))
                         : (p.acc ? launch_aa_tma<DT, false, true>(p, a, s) : launch_aa_tma<DT, false, false>(p, a, s));
       if (e != cudaErrorNotSupported) return e;
     }
   }
-  if constexpr (is16(DT)) {                          // no tensor maps: the same step from the lattice
+  if constexpr (is16(DT)) {                          // the same step from the lattice
     using Cfg = StepCfg<4, 8>;
     const dim3 grid((unsigned)((p.g.nseg_x + 1) / 2), (unsigned)((p.g.ny + Cfg::WY - 1) / Cfg::WY), (unsigned)p.g.nz);
     const dim3 block(32, Cfg::WY);
