@@ -36,7 +36,7 @@ def _download(t):
     """A device tensor as a NumPy array.  The pages of a large array that was just allocated are
     touched by all host threads first: mapped one by one under the copy they cost four times the
     copy itself (336 MB: 11.6 ms, 4.4 ms this way)."""
-    out = torch.empty(t.shape, dtype=t.dtype)
+    out = torch.empty(t.shape, dtype=t.dtype, device="cpu")
     if out.numel() * out.element_size() >= 1 << 22:
         out.fill_(0)
     return out.copy_(t).numpy()
