@@ -82,9 +82,6 @@ template <typename T> __device__ __forceinline__ void st_new(T *q, T v, const Ho
 __device__ __forceinline__ void st_new(float *q, float v, const Hold<true> &h) {
   asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(q), "f"(v), "l"(h.policy) : "memory");
 }
-__device__ __forceinline__ void st_new(double *q, double v, const Hold<true> &h) {
-  asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;" ::"l"(q), "d"(v), "l"(h.policy) : "memory");
-}
 __device__ __forceinline__ void st_new(unsigned int *q, unsigned int v, const Hold<true> &h) {
   asm volatile("st.global.L2::cache_hint.b32 [%0], %1, %2;" ::"l"(q), "r"(v), "l"(h.policy) : "memory");
 }
