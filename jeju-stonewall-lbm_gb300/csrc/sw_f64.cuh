@@ -5,9 +5,10 @@
 // alike) against 64 integer ones: the collision's 206 double operations take
 // 3300 clocks per warp, seven times what its 304 bytes per cell take at the
 // measured HBM rate.  So the cell's tensors are held as 64-bit integers in
-// units of 2^-62 and only the scalar functions (1 / rho, the two square roots
-// of the Smagorinsky time scale, 1 / tau) stay in double: 23 double operations
-// per cell beside about 500 integer ones, which run on other pipes.
+// units of 2^-62 and only the scalar functions stay in double: 1 / rho and
+// 1 / tau (three operations each), the two square roots of the Smagorinsky time
+// scale (five each), three products and sums and the sponge's four, 23 per cell
+// beside about 500 integer ones, which run on other pipes.
 //
 //  * A population in [2^-10, its limit below 1/2) is a whole number of units, so
 //    the conversion is exact, and so are rho, m and Pi: sums of 19 exact terms,
@@ -21,8 +22,8 @@
 //    additions, shifts and four multiplications by constants.
 //  * The results are rounded to double once, at the end.
 // Cells with a population outside its range (also negative ones, infinities and
-// NaN), rho outside [1/2, 2), or a result outside [2^-10, 1) report so and the
-// caller collides them in double.
+// NaN), rho outside (1/2, 2), 1 / tau outside [1/4, 2] or a result outside
+// [2^-10, 1) report so and the caller collides them in double.
 //
 // Error of one collision against 128-bit floats on the same inputs (25 kinds of
 // 20 000 cells, |u_a| up to 0.25, |Pi_neq| up to 3e-2): 4.6e-17 to 5.5e-17 of the
@@ -204,7 +205,8 @@ __host__ __device__ __forceinline__ bool collide(const double (&f)[19], double t
     return (i64)(int)vh * (int)vh + (((i64)(int)vh * (int)(vl >> 1)) >> 30);
   };
   const i64 q = (square(nxx) + square(nyy) + square(nzz)) + ((square(nxy) + square(nxz) + square(nyz)) << 1);
-  // below 2^40 only where every entry is below 2^-30: |Pi_neq| then counts as 2^-39, far below tau0's last place
+  // below 2^40 only where every entry is below 2^-39: |Pi_neq| then counts as 2^-39, which moves tau by about 2^-40
+  // and what it multiplies, those entries, by 2^-79
   const uint32_t qh = hi32((u64)q) < 256u ? 256u : hi32((u64)q);
   const double qn = scaled(square_root(of_units(join(qh, lo32((u64)q)))), 1 - lead);
   const double root = square_root(dfma(dmul(c18, y), qn, tau0sq));
