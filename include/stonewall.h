@@ -147,8 +147,8 @@ int sw_step_accum(const sw_geom *g, int dtype, const void *f_in, void *f_out, co
  * 8-17 two cells per thread with TMA-staged sources (csrc/sw_tma.cuh), the
  * last two groups for 16-bit storage only; they round alike, and unlike 0-3.  sw_step and sw_step_accum use the
  * configuration set for their storage type (process-wide, default 0);
- * stonewall/autotune.py times those that round alike (4-17 for 16-bit storage)
- * and sets the fastest.  No reference counterpart (Warp chooses its own launch shape). */
+ * stonewall/autotune.py times those that round alike (for 16-bit storage 4-17, or
+ * 0-3 for the accumulating steps of some grids) and sets the fastest.  No reference counterpart (Warp chooses its own launch shape). */
 int sw_step_config_count(void);
 /* Blocks of the TMA-staged configurations that gave up a bounded wait for
  * their copies since the last call (read and cleared; -1 if unreadable).  A

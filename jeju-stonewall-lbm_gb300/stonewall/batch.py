@@ -305,7 +305,7 @@ class Batch:
             # two-lattice members' configurations are still tuned on the largest of them
             ab = [m for m in self.pending() if getattr(m, "pattern", "ab") == "ab"]
             if ab:
-                single.tune(max(ab, key=lambda m: m.grid.cells))
+                single.tune(max(ab, key=lambda m: m.grid.cells), alone=False)
             self.mode = "graph"
             return "graph", times
         if "persistent" in modes:
@@ -326,7 +326,7 @@ class Batch:
             self.cfg = min(times, key=times.get)
         live = self.pending()
         if "graph" in modes and 0 < len(live) <= GRAPH_MAX:
-            single.tune(max(live, key=lambda m: m.grid.cells))
+            single.tune(max(live, key=lambda m: m.grid.cells), alone=False)
             slot, lv = self._fill(1, tuning=True, upload=False)
             self._graph_run(slot, len(lv), 1)                       # instantiate
             torch.cuda.synchronize()

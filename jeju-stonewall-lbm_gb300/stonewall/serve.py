@@ -109,6 +109,7 @@ def make_solver(req, p, flag, device="cuda", pattern="ab"):
                    device=device, pattern=pattern)
     s.init(noise=0.02, seed=req.seed, noise_kind="gauss")
     s.params = p
+    s.shares_tuning = True           # the server tunes a storage type once, on whichever wall comes first
     return s
 
 

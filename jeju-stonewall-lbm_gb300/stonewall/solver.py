@@ -121,6 +121,7 @@ class WallSolver:
         self.t = 0
         self.n_acc = 0
         self.chunk = int(chunk)
+        self.shares_tuning = False   # autotune(): its choice also serves walls of other sizes
         self._graphs = {}
         self._q_levels = (None, None)   # quantisation levels of q_frame on the device, for one qmax
         self._ring = None
@@ -175,7 +176,7 @@ class WallSolver:
         from . import autotune
         if self.pattern == "aa":
             return N.lib().sw_get_step_config(self.dtype), {}   # the in-place step has one configuration
-        return autotune.tune(self, repeats=repeats)
+        return autotune.tune(self, repeats=repeats, alone=not self.shares_tuning)
 
     def init(self, noise=0.02, seed=7, noise_kind="uniform"):
         """k_init on the current lattice (lbm3d.py:340); clears the status word."""
