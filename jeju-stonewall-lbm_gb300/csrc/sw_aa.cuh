@@ -735,9 +735,15 @@ __device__ __forceinline__ void aa_odd_pair_checked(const StepParams &p, const u
   if (force && p.force != nullptr) warp_force_add<float>(p, z, lane, fxw, fzw, hit);
 }
 
+// The tensor maps of a step: the even step's only copy takes all populations.
+struct OwnMap {
+  CUtensorMap one;
+};
+template <bool ODD> using AAMapsOf = std::conditional_t<ODD, LatticeMaps, OwnMap>;
+
 template <int DT, bool ODD, bool ACC, bool KEEP>
 __global__ void __launch_bounds__(128, 9)
-    k_step_aa_tma(const __grid_constant__ LatticeMaps maps, const __grid_constant__ CUtensorMap map_acc,
+    k_step_aa_tma(const __grid_constant__ AAMapsOf<ODD> maps, const __grid_constant__ CUtensorMap map_acc,
                   const __grid_constant__ StepParams p, AAParams a) {
   using PK = Pack16<DT>;
   extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -753,7 +759,7 @@ __global__ void __launch_bounds__(128, 9)
     mbar_init(smem_u32(&bar), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    if (ODD) tma_issue<ACC>(maps, &map_acc, g, x0s, y0, z, st, smem_u32(&bar));
+    if constexpr (ODD) tma_issue<ACC>(maps, &map_acc, g, x0s, y0, z, st, smem_u32(&bar));
     else tma_issue_own<ACC>(&maps.one, &map_acc, x0s, y0, z, st, smem_u32(&bar));
   }
   const int sa = 2 * bx;
@@ -891,15 +897,19 @@ template <int DT> inline bool hold_aa(const StepParams &p) {
   return DT == SW_F32 && (p.acc != nullptr || bytes < 112000000ll);
 }
 
+inline bool encode_lattice_maps(OwnMap *m, const void *f, const Geom &g) { return encode_lattice_map(&m->one, f, g, 4, Q); }
+
 // The TMA-staged AA step on the lattice p.fin (== p.fout); cudaErrorNotSupported
-// when the tensor maps cannot be made (the caller then runs k_step_aa_pair).
+// when the tensor maps cannot be made (the caller then runs k_step_aa_pair).  The odd
+// step groups its copies at every size (us per step, odd and even together, one copy per
+// population / grouped: alone H 5 10.6 / 10.6, H 8 12.45 / 12.36, H 16 26.1 / 25.9, H 24
+// 86.9 / 86.2, H 40 321 / 318; three walls side by side in one graph H 5 16.4 / 17.0,
+// H 8 22.1 / 23.0, H 12 39.7 / 40.2, H 16 76.0 / 75.7, H 24 257 / 256).
 template <int DT, bool ODD, bool ACC>
 cudaError_t launch_aa_tma(const StepParams &p, const AAParams &a, cudaStream_t s) {
-  LatticeMaps maps;
+  AAMapsOf<ODD> maps;
   CUtensorMap map_acc;
-  // the even step's only copy takes all populations (in `one`)
-  if (ODD ? !encode_lattice_maps(&maps, p.fin, p.g) : !encode_lattice_map(&maps.one, p.fin, p.g, 4, Q))
-    return cudaErrorNotSupported;
+  if (!encode_lattice_maps(&maps, p.fin, p.g)) return cudaErrorNotSupported;
   if (ACC) {
     if (!encode_acc_map(&map_acc, p.acc, p.g)) return cudaErrorNotSupported;
   } else {
