@@ -30,7 +30,7 @@ def config_count():
 
 def one_cell_sums(grid):
     """Whether accumulating steps of a 16-bit wall of this grid run one cell per thread.  They do from
-    where the two-cell blocks (64 cells of 4 rows) need a second round on the 152 SMs, eight to each,
+    where the two-cell blocks (64 cells of 4 rows) need a second wave on the 152 SMs, eight to each,
     which the shorter blocks fill better, up to where lattices, sums and flags leave the L2 and the
     wider accesses win (captured graphs, us per step, one cell / two: 1080 blocks 10.03 / 9.52, 1216
     10.11 / 10.83, 1230 10.43 / 10.11, 1360 10.33 / 10.82, 2040 11.9 / 14.2, 3000 15.0 / 18.3; 93 MB
